@@ -32,6 +32,7 @@
 
 namespace gk {
 
+constexpr int64_t CM_ROW_LIMIT = int64_t(1) << 31;  // products of a row (counts within a row are 32-bit)
 constexpr int CM_WARP_WORK = 256, CM_CTA_WORK = 2048;  // products of the hash classes
 // A window's CTA: 128 threads where a row's window is small, so that many rows
 // are in flight (a row is a chain of a dozen dependent loads and barriers:
@@ -48,6 +49,7 @@ struct CmaskState {
     unsigned int n[3];      // rows of each class
     unsigned int fetch[3];  // next row of each class
     unsigned int mismatch;  // C_rowptr is not this product's
+    unsigned int too_long;  // a row has CM_ROW_LIMIT products or more
 };
 
 struct CmaskArgs {
@@ -80,6 +82,10 @@ __global__ void __launch_bounds__(256) k_cmask_classes(CmaskArgs a) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xFFFFFFFFu, w, o);
         if (lane != 0) continue;
+        if (w >= CM_ROW_LIMIT) {
+            a.st->too_long = 1;
+            continue;
+        }
         if (w == 0) {
             if (a.cnt) a.cnt[i] = 0;
             else if (a.crp[i + 1] != a.crp[i]) a.st->mismatch = 1;
@@ -460,6 +466,7 @@ extern "C" int gk_mxmm_cmask(const gk_csr *A, const gk_csr *B, const gk_csr *M, 
         GK_CHECK(check_csr(a.M, CSR_SORTED, "M", s, scr));
         return fail(GK_ERR_INVALID_CSR, "defect found by the content check");
     }
+    if (h.too_long) return fail(GK_ERR_UNSUPPORTED, "complement-masked product: a row has >= 2^31 products");
     if (fill) {
         if (ends[0] != 0) return fail(GK_ERR_ARG, "C_rowptr[0] must be 0 (pass the first call's row pointers)");
         if (h.mismatch)

@@ -78,3 +78,22 @@ def test_foreign_row_pointers(gk, cuda):
                                col.ctypes.data, val.ctypes.data, None)
         assert rc == gk._lib.GK_ERR_ARG
         assert (col[n:] == -7).all() and (val[n:] == -7).all()
+
+
+@pytest.mark.parametrize("entries", [5000, 1 << 19])
+def test_row_of_too_many_products(gk, cuda, entries):
+    """A row of 2^31 products is refused, a shorter one is not (A's order and
+    duplicates do not matter)."""
+    n, b = 1 << 15, 1 << 12
+    A = G.Csr(2, 1, np.array([0, 1, 1 + entries]), np.zeros(1 + entries, dtype=np.int32), None)
+    B = G.Csr(1, n, np.array([0, b]), np.arange(b, dtype=np.int32) * 3, None)
+    M = G.Csr(2, n, np.array([0, 0, 1]), np.array([6], dtype=np.int32), None)
+    if entries * b < 1 << 31:
+        C = gk.mxmm_cmask(A.to("cuda"), B.to("cuda"), M.to("cuda"), semiring="plus_pair").numpy()
+        np.testing.assert_array_equal(C.rowptr, [0, b, 2 * b - 1])
+        np.testing.assert_array_equal(C.col[b:], np.delete(np.arange(b) * 3, 2))
+        np.testing.assert_array_equal(C.val, [1] * b + [entries] * (b - 1))
+    else:
+        with pytest.raises(gk.GkError) as e:
+            gk.mxmm_cmask(A.to("cuda"), B.to("cuda"), M.to("cuda"), semiring="plus_pair")
+        assert e.value.code == gk._lib.GK_ERR_UNSUPPORTED
