@@ -15,6 +15,9 @@
 //                         products set bits, M's row clears them, and prefix
 //                         counts over the words give every column its place, at
 //                         which a second reading of the products adds them up
+// Such a row costs at least its windows, whatever it holds: calls with several
+// windows a row and too few products for them take the sort of cmask_sort.cu
+// (cm_sorts).
 // A's entries are taken 32 at a time per warp and their B rows' elements packed
 // onto the lanes, so that short B rows leave no lanes idle.  Nothing is written
 // to memory but C itself: expanding all products as 64-bit keys, sorting and
@@ -27,6 +30,7 @@
 
 #include <algorithm>
 
+#include "gk_cmask.cuh"
 #include "gk_common.cuh"
 #include "gk_device.cuh"
 
@@ -50,6 +54,7 @@ struct CmaskState {
     unsigned int fetch[3];  // next row of each class
     unsigned int mismatch;  // C_rowptr is not this product's
     unsigned int too_long;  // a row has CM_ROW_LIMIT products or more
+    unsigned long long work, long_work, max_work;  // products: all, those of rows in windows, the longest row's
 };
 
 struct CmaskArgs {
@@ -59,6 +64,7 @@ struct CmaskArgs {
     int64_t *cnt;        // symbolic call: entries of every row
     int32_t *c_col, *c_val;
     uint32_t *rows;  // three lists of up to m rows
+    int64_t *work;   // products of every row, where cm_sorts may want them (else null)
     CmaskState *st;
     int checked;  // the checks ran: nothing is read through a matrix that one of them refused
     int win;      // log2 columns of a window
@@ -73,6 +79,7 @@ __global__ void __launch_bounds__(256) k_cmask_classes(CmaskArgs a) {
     if (!a.ready()) return;
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    unsigned long long all = 0, in_windows = 0, longest = 0;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.A.m; i += warps) {
         int64_t w = 0;
         for (int64_t t = a.A.rp[i] + lane; t < a.A.rp[i + 1]; t += 32) {
@@ -82,6 +89,7 @@ __global__ void __launch_bounds__(256) k_cmask_classes(CmaskArgs a) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xFFFFFFFFu, w, o);
         if (lane != 0) continue;
+        if (a.work) a.work[i] = w;
         if (w >= CM_ROW_LIMIT) {
             a.st->too_long = 1;
             continue;
@@ -95,6 +103,14 @@ __global__ void __launch_bounds__(256) k_cmask_classes(CmaskArgs a) {
         // from a warp's work on
         const int c = w <= CM_WARP_WORK ? 0 : (w <= CM_CTA_WORK && a.B.n > (1 << 15) ? 1 : 2);
         a.rows[c * a.A.m + atomicAdd(&a.st->n[c], 1u)] = static_cast<uint32_t>(i);
+        all += w;
+        if (c == 2) in_windows += w;
+        longest = max(longest, static_cast<unsigned long long>(w));
+    }
+    if (a.work && all) {
+        atomicAdd(&a.st->work, all);
+        atomicAdd(&a.st->long_work, in_windows);
+        atomicMax(&a.st->max_work, longest);
     }
 }
 
@@ -377,11 +393,45 @@ static int launch_map(const CmaskArgs &a, cudaStream_t s) {
     return GK_OK;
 }
 
-template <bool FILL>
-static int launch_rows(const CmaskArgs &a, cudaStream_t s) {
+static int launch_classes(const CmaskArgs &a, cudaStream_t s) {
     k_cmask_classes<<<ctx().num_sms * 8, 256, 0, s>>>(a);
     note_launches(1);
     GK_CUDA(cudaGetLastError());
+    return GK_OK;
+}
+
+// Whether the sort is the better path for these rows: the estimates of both calls'
+// times in us, fitted to the figures below (2^18 columns or fewer: never).  A row in
+// windows costs 0.72 us a window spread over the SMs (clearing, counting and writing
+// 2^14 words) and at least one SM's share of that, 9 us per million products a
+// window, hashed rows 120; the sort 0.8 ms and 260 us per million products, and in
+// every batch of 2^26 products the warp of the longest row is waited for (20 ms per
+// million of its products).  ms, windows / sort, rows x products at columns:
+//   20,000 x 2,400 at 2^19  15.4 / 11.8   2,000 x 3,000 at 2^20   3.6 / 2.2
+//   20,000 x 4,500 at 2^19  17.3 / 23     2,000 x 3,000 at 2^24  47.4 / 2.2
+//   20,000 x 12,000 at 2^20 35.8 / 66     2,000 x 30,000 at 2^24 62.4 / 15.3
+//   5,000 x 40,000 at 2^21  27.8 / 71       200 x 500,000 at 2^24  51 / 105
+constexpr int CM_SORT_WIN = 19;  // windows from which the question is asked
+static bool cm_sorts(const CmaskState &st, int64_t n, int win, int sms) {
+    if (st.n[2] == 0) return false;
+    const double windows = static_cast<double>((n + (int64_t(1) << win) - 1) >> win);
+    const double rows = std::max<double>(st.n[2], sms), work = static_cast<double>(st.work);
+    const double by_windows = windows * (0.72 * rows + 9e-6 * st.long_work) + 1.2e-4 * (work - st.long_work);
+    const double batches = std::max(1.0, work / double(1 << 26));
+    const double by_sort = 800.0 + 2.6e-4 * work + 2.0 * batches * 0.02 * st.max_work;
+    return by_sort < by_windows;
+}
+
+// All rows of a, read from its state as ready, by the sort.
+static int cmask_by_sort(const CmaskArgs &a, cudaStream_t s, Scratch &scr) {
+    int64_t *cnt = a.cnt;
+    if (!cnt) GK_CHECK(scr.alloc(&cnt, a.A.m + 1));  // numeric call
+    return cmask_by_sort(a.A, a.B, a.M, a.values, a.work, cnt, a.crp, a.crp ? a.c_col : nullptr, a.c_val,
+                         &a.st->mismatch, s, scr);
+}
+
+template <bool FILL>
+static int launch_rows(const CmaskArgs &a, cudaStream_t s) {
     // the longest rows first
     if (FILL && a.win <= CM_DENSE_WIN) GK_CHECK((launch_map<256, FILL, FILL>(a, s)));
     else if (a.win <= CM_SMALL_WIN) GK_CHECK((launch_map<128, FILL, false>(a, s)));
@@ -451,22 +501,39 @@ extern "C" int gk_mxmm_cmask(const gk_csr *A, const gk_csr *B, const gk_csr *M, 
         }
         a.c_col = dcol;
         a.c_val = dval;
-        if (m > 0) GK_CHECK(launch_rows<true>(a, s));
     } else {
         GK_CHECK(scr.alloc(&a.cnt, m + 1));
         GK_CUDA(cudaMemsetAsync(a.cnt + m, 0, sizeof(int64_t), s));
-        if (m > 0) GK_CHECK(launch_rows<false>(a, s));
     }
+    const bool may_sort = m > 0 && a.win >= CM_SORT_WIN;
+    if (may_sort) GK_CHECK(scr.alloc(&a.work, m));
     CmaskState h{};
-    GK_CUDA(cudaMemcpyAsync(&h, a.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    GK_CUDA(cudaStreamSynchronize(s));
-    if (check && !(h.chk[0].sound() && h.chk[1].sound() && h.chk[2].sound())) {
-        GK_CHECK(check_csr(a.A, CSR_STRUCTURE, "A", s, scr));  // names the defect
-        GK_CHECK(check_csr(a.B, CSR_STRUCTURE, "B", s, scr));
-        GK_CHECK(check_csr(a.M, CSR_SORTED, "M", s, scr));
-        return fail(GK_ERR_INVALID_CSR, "defect found by the content check");
+    auto read_state = [&]() -> int {  // its defects, too
+        GK_CUDA(cudaMemcpyAsync(&h, a.st, sizeof(h), cudaMemcpyDeviceToHost, s));
+        GK_CUDA(cudaStreamSynchronize(s));
+        if (check && !(h.chk[0].sound() && h.chk[1].sound() && h.chk[2].sound())) {
+            GK_CHECK(check_csr(a.A, CSR_STRUCTURE, "A", s, scr));  // names the defect
+            GK_CHECK(check_csr(a.B, CSR_STRUCTURE, "B", s, scr));
+            GK_CHECK(check_csr(a.M, CSR_SORTED, "M", s, scr));
+            return fail(GK_ERR_INVALID_CSR, "defect found by the content check");
+        }
+        if (h.too_long) return fail(GK_ERR_UNSUPPORTED, "complement-masked product: a row has >= 2^31 products");
+        return GK_OK;
+    };
+    if (m > 0) GK_CHECK(launch_classes(a, s));
+    if (may_sort) GK_CHECK(read_state());
+    bool done = m == 0;
+    if (may_sort && cm_sorts(h, B->n, a.win, ctx().num_sms)) {
+        if (fill && ends[0] != 0)
+            return fail(GK_ERR_ARG, "C_rowptr[0] must be 0 (pass the first call's row pointers)");
+        // without room for the products (nothing is written before it is known) the windows serve
+        Scratch own(s);
+        const int status = cmask_by_sort(a, s, own);
+        if (status != GK_ERR_OOM) GK_CHECK(status);
+        done = status == GK_OK;
     }
-    if (h.too_long) return fail(GK_ERR_UNSUPPORTED, "complement-masked product: a row has >= 2^31 products");
+    if (!done) GK_CHECK(fill ? launch_rows<true>(a, s) : launch_rows<false>(a, s));
+    GK_CHECK(read_state());
     if (fill) {
         if (ends[0] != 0) return fail(GK_ERR_ARG, "C_rowptr[0] must be 0 (pass the first call's row pointers)");
         if (h.mismatch)

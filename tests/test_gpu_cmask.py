@@ -97,3 +97,68 @@ def test_row_of_too_many_products(gk, cuda, entries):
         with pytest.raises(gk.GkError) as e:
             gk.mxmm_cmask(A.to("cuda"), B.to("cuda"), M.to("cuda"), semiring="plus_pair")
         assert e.value.code == gk._lib.GK_ERR_UNSUPPORTED
+
+
+def random_rows(m, n, per_row, seed, values=True):
+    rng = np.random.default_rng(seed)
+    return csr(m, n, np.repeat(np.arange(m), per_row), rng.integers(0, n, m * per_row), seed, values)
+
+
+def test_long_rows_over_very_many_columns(gk, orc, cuda):
+    """Rows of some thousand products over 2^23 columns, which are sorted (in
+    windows where that finds no memory), among short and empty ones."""
+    n, k = (1 << 23) + 5, 2000
+    A = csr(60, k, np.concatenate([np.repeat(np.arange(40), 90), np.arange(40, 58)]),
+            np.random.default_rng(1).integers(0, k, 3618), 1)
+    B, M = random_rows(k, n, 40, 2), random_rows(60, n, 30, 3, values=False)
+    M = csr(60, n, np.concatenate([np.repeat(np.arange(60), np.diff(M.rowptr)), np.arange(4000) % 60]),
+            np.concatenate([M.col, B.col[:4000]]), 4, values=False)
+    rp, col, val = orc.mxmm_cmask(A, B, M)
+    dev = [x.to("cuda") for x in (A, B, M)]
+    lib = gk.load()
+    failures = 0
+    for after in [-1] + list(range(40)):
+        lib.gk_inject_alloc_failure(after)
+        try:
+            C = gk.mxmm_cmask(*dev).numpy()
+        except gk.GkError as e:
+            assert e.code == gk._lib.GK_ERR_OOM
+            failures += 1
+            continue
+        finally:
+            lib.gk_inject_alloc_failure(-1)
+        np.testing.assert_array_equal(C.rowptr, rp)
+        np.testing.assert_array_equal(C.col, col)
+        np.testing.assert_array_equal(C.val, val)
+    assert failures < 12  # the calls' own few arrays
+    # foreign row pointers
+    ga, gb, gm = (x.as_gk() for x in (A, B, M))
+    for bad in (np.concatenate([rp[:3], rp[3:] + 1]), np.concatenate([rp[:-1] * 0, rp[-1:]]),
+                np.concatenate([rp[:5], rp[4:5], rp[6:]])):
+        bad = np.ascontiguousarray(bad, dtype=np.int64)
+        c, v = np.full(int(bad[-1]) + 64, -7, dtype=np.int32), np.full(int(bad[-1]) + 64, -7, dtype=np.int32)
+        rc = lib.gk_mxmm_cmask(ctypes.byref(ga), ctypes.byref(gb), ctypes.byref(gm), 0, bad.ctypes.data, c.ctypes.data,
+                               v.ctypes.data, None)
+        assert rc == gk._lib.GK_ERR_ARG
+        assert (c[int(bad[-1]):] == -7).all() and (v[int(bad[-1]):] == -7).all()
+
+
+def test_time_does_not_grow_with_the_columns(gk, cuda):
+    """The same number of products over 2^24 columns took 60 times as long as over
+    2^17, window by window; the sort takes some three times as long."""
+    import torch
+
+    def best(n):
+        args = [x.to("cuda") for x in (random_rows(2000, 20000, 100, 5), random_rows(20000, n, 30, 6),
+                                       random_rows(2000, n, 20, 7, values=False))]
+        ts = []
+        for _ in range(5):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            gk.mxmm_cmask(*args)
+            t1.record()
+            torch.cuda.synchronize()
+            ts.append(t0.elapsed_time(t1))
+        return min(ts)
+
+    assert best(1 << 24) < 15 * best(1 << 17)
