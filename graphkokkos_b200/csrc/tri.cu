@@ -931,10 +931,57 @@ struct TriGate {
 constexpr int64_t TRI_SMALL_M = 65536;  // vertices: a bitmap of a row's columns fits the warp's shared memory
 constexpr int TRI_SMALL_WARPS = 4;
 
+// Whether x is among the n ascending columns of c.
+__device__ __forceinline__ bool tri_small_has(const int32_t *__restrict__ c, uint32_t n, int x) {
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t md = (lo + hi) >> 1;
+        if (__ldg(c + md) < x) lo = md + 1;
+        else hi = md;
+    }
+    return lo < n && __ldg(c + lo) == x;
+}
+
+// Hits of a row L_i (ri, len columns) in the rows L_k of up to 32 entries (one per
+// lane: n columns from col + b0) without its bitmap: an L_k far longer than L_i is
+// searched for L_i's columns, the others' columns are searched for in L_i.
+constexpr uint32_t TRI_SMALL_UNEVEN = 32;
+__device__ __forceinline__ bool tri_small_longer(uint32_t n, uint32_t len) { return n > TRI_SMALL_UNEVEN * (len + 32); }
+
+__device__ __forceinline__ uint32_t tri_small_search(const int32_t *__restrict__ col, const int32_t *__restrict__ ri,
+                                                  uint32_t len, int64_t b0, uint32_t n) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const bool longer = tri_small_longer(n, len);
+    uint32_t cnt = 0;
+    for (unsigned todo = __ballot_sync(FULL, longer); todo; todo &= todo - 1) {
+        const int j = __ffs(todo) - 1;
+        const int64_t bj = __shfl_sync(FULL, b0, j);
+        const uint32_t nj = __shfl_sync(FULL, n, j);
+        for (uint32_t q = lane; q < len; q += 32) cnt += tri_small_has(col + bj, nj, __ldg(ri + q));
+    }
+    const uint32_t m = longer ? 0 : n, incl = warp_incl_sum(m, lane), total = __shfl_sync(FULL, incl, 31);
+    for (uint32_t b = 0; b < total; b += 32) {
+        const uint32_t at = b + lane;
+        const int j = warp_find(incl, at) & 31;
+        const int64_t q = __shfl_sync(FULL, b0, j) + (at - __shfl_sync(FULL, incl - m, j));
+        if (at < total) cnt += tri_small_has(ri, len, __ldg(col + q));
+    }
+    return cnt;
+}
+
 // Sum of C<L> = L·L.  A warp takes 32 entries of L at a time; for each row i
 // among them the columns of L_i go to a bitmap in shared memory, and the rows
 // L_k of the entries k are read four columns per lane and tested.  No plan: the
 // entries, not the rows, are dealt out, so a hub row is spread over warps.
+// Very uneven pairs take the search above, since a warp would read a whole long row
+// for a few columns: the bitmap of a long L_i whose L_k hold little (16,384
+// vertices, 32 rows of all columns: 1.20 -> 0.05 ms), or an L_k far longer than L_i
+// (65,536 vertices, one row of 32,768 columns named by as many rows: 3.35 -> 0.10
+// ms).  The ordinary rows' loads are left as they were, the bitmap's in flight with
+// those of the L_k (bitmap only once the L_k's columns are counted: RMAT-16 340 ->
+// 490 us; the search out of line: RMAT-8 45 -> 48 us, in line 43).
+constexpr uint32_t TRI_SMALL_MAP = 1024;  // columns of an L_i that is mapped in any case
 __global__ void __launch_bounds__(32 * TRI_SMALL_WARPS) k_tri_small(DevCsr L, int words, TriGate gate,
                                                                     unsigned long long *sum) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -971,11 +1018,23 @@ __global__ void __launch_bounds__(32 * TRI_SMALL_WARPS) k_tri_small(DevCsr L, in
                     b0 = __ldg(L.rp + k);
                     n = static_cast<uint32_t>(__ldg(L.rp + k + 1) - b0);
                 }
+                const uint32_t len = static_cast<uint32_t>(r1 - r0);
+                p = e;
+                if (len > TRI_SMALL_MAP && 8 * __reduce_add_sync(FULL, min(n, 1u << 16)) < len) {
+                    cnt += tri_small_search(L.col, L.col + r0, len, b0, n);
+                    r0 = r1;
+                    continue;
+                }
                 for (int64_t q = r0 + lane; q < r1; q += 32) {
                     const int x = __ldg(L.col + q);
                     atomicOr(bm + (x >> 5), 1u << (x & 31));
                 }
                 __syncwarp();
+                const bool longer = tri_small_longer(n, len);
+                if (__any_sync(FULL, longer)) {
+                    cnt += tri_small_search(L.col, L.col + r0, len, b0, longer ? n : 0);
+                    if (longer) n = 0;
+                }
                 const uint32_t u = (n + 3) / 4, incl = warp_incl_sum(u, lane);
                 const uint32_t total = __shfl_sync(FULL, incl, 31);
                 for (uint32_t b = 0; b < total; b += 32) {
@@ -996,7 +1055,6 @@ __global__ void __launch_bounds__(32 * TRI_SMALL_WARPS) k_tri_small(DevCsr L, in
                 __syncwarp();
                 for (int64_t q = r0 + lane; q < r1; q += 32) bm[__ldg(L.col + q) >> 5] = 0;
                 __syncwarp();
-                p = e;
             }
             r0 = r1;
         }
