@@ -577,37 +577,64 @@ int gk_tc_count_batched(const gk_csr *graphs, int ngraphs, uint64_t *counts, int
         GK_CUDA(cudaStreamSynchronize(s));
         const auto walked = [&](const GraphSlot &x) { return per[x.id] < TRI_WALK_WORK_BATCH; };
         nwalk = static_cast<int>(std::stable_partition(slots.begin(), slots.end(), walked) - slots.begin());
+    }
+    GraphSlot *dslots;
+    GK_CHECK(scr.alloc(&dslots, ngraphs));
+    // per-graph entry ranges for the content check, and its flags
+    // (and every graph's first vertex)
+    std::vector<int64_t> ranges(3 * static_cast<size_t>(ngraphs));
+    int64_t *dranges;
+    unsigned int *bad;
+    GK_CHECK(scr.alloc(&dranges, ranges.size()));
+    const int64_t *dvbase = dranges + 2 * static_cast<size_t>(ngraphs);
+    GK_CHECK(scr.alloc(&bad, 1));
+    // places of the graphs in the combined matrix, in the order of the slots
+    auto place = [&]() -> int {
         int64_t v = 0, e = 0;
         for (GraphSlot &x : slots) {
             x.vbase = v;
             x.ebase = e;
             v += x.m;
             e += x.nnz;
+            ranges[2 * x.id] = x.ebase;
+            ranges[2 * x.id + 1] = x.ebase + x.nnz;
+            ranges[2 * static_cast<size_t>(ngraphs) + x.id] = x.vbase;
         }
-    }
-    GraphSlot *dslots;
-    GK_CHECK(scr.alloc(&dslots, ngraphs));
-    GK_CUDA(cudaMemcpyAsync(dslots, slots.data(), sizeof(GraphSlot) * ngraphs, cudaMemcpyHostToDevice, s));
-    // per-graph entry ranges for the content check, and its flags
-    // (and every graph's first vertex)
-    std::vector<int64_t> ranges(3 * static_cast<size_t>(ngraphs));
-    for (const GraphSlot &x : slots) {
-        ranges[2 * x.id] = x.ebase;
-        ranges[2 * x.id + 1] = x.ebase + x.nnz;
-        ranges[2 * static_cast<size_t>(ngraphs) + x.id] = x.vbase;
-    }
-    int64_t *dranges;
-    unsigned int *bad;
-    GK_CHECK(scr.alloc(&dranges, ranges.size()));
-    const int64_t *dvbase = dranges + 2 * static_cast<size_t>(ngraphs);
-    GK_CHECK(scr.alloc(&bad, 1));
-    GK_CUDA(cudaMemcpyAsync(dranges, ranges.data(), sizeof(int64_t) * ranges.size(), cudaMemcpyHostToDevice, s));
-    GK_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), s));
+        GK_CUDA(cudaMemcpyAsync(dslots, slots.data(), sizeof(GraphSlot) * ngraphs, cudaMemcpyHostToDevice, s));
+        GK_CUDA(cudaMemcpyAsync(dranges, ranges.data(), sizeof(int64_t) * ranges.size(), cudaMemcpyHostToDevice, s));
+        GK_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), s));
+        return GK_OK;
+    };
+    GK_CHECK(place());
+    // graphs [g0, g1) of the slots into the combined matrix
+    auto concat = [&](int g0, int g1, int64_t vend, int64_t eend) -> int {
+        int64_t largest = 0;
+        for (int g = g0; g < g1; ++g) largest = std::max(largest, slots[g].nnz);
+        // CTAs a graph: enough that the largest graph's share is a few steps each
+        const dim3 grid(g1 - g0, static_cast<unsigned>(std::min<int64_t>(std::max<int64_t>(largest >> 14, 8), 64)));
+        k_concat_graphs<<<grid, 256, 0, s>>>(dslots + g0, rp, col, key, bad);
+        k_set_last<<<1, 1, 0, s>>>(rp, vend, eend);  // the group's end (the next group writes the same value)
+        note_launches(2);
+        GK_CUDA(cudaGetLastError());
+        return GK_OK;
+    };
+    // The first bad row of graphs in two groups, numbered in the caller's order: all
+    // of them are laid out and checked again, in that order.
+    auto caller_defect = [&]() -> int {
+        if (nwalk == 0 || nwalk == ngraphs) return GK_OK;
+        std::sort(slots.begin(), slots.end(), [](const GraphSlot &a, const GraphSlot &b) { return a.id < b.id; });
+        GK_CHECK(place());
+        GK_CHECK(concat(0, ngraphs, vtot, etot));
+        Scratch cs(s);
+        return check_csr_batch(DevCsr{vtot, vtot, etot, rp, col, nullptr}, 0, 0, key, dranges, bad, CSR_SORTED,
+                               "graphs", s, cs);
+    };
 
     // Groups of consecutive graphs.  With host inputs the copies of group q+1
     // run on a side stream while group q is counted (the graphs are
-    // independent, so a group needs only its own rows).  A group holds about etot/8 entries, at least GK_BATCH_STAGE_MIN
-    // (default 2^24, whose copy takes ~1 ms).  All copies are queued at once,
+    // independent, so a group needs only its own rows).  A group holds about
+    // etot/8 entries, at least GK_BATCH_STAGE_MIN (default 2^24, whose copy takes
+    // ~1 ms).  All copies are queued at once,
     // so they run back to back while the counts follow them group by group.
     // (Groups that double in size, which expose only a small first copy, were
     // slower on the uneven 4,096-graph batch: its compute-light Erdos-Renyi
@@ -650,14 +677,7 @@ int gk_tc_count_batched(const gk_csr *graphs, int ngraphs, uint64_t *counts, int
         }
         const int64_t v0 = slots[g0].vbase, e0 = slots[g0].ebase;
         const int64_t v1 = g1 < ngraphs ? slots[g1].vbase : vtot, e1 = g1 < ngraphs ? slots[g1].ebase : etot;
-        int64_t largest = 0;
-        for (int g = g0; g < g1; ++g) largest = std::max(largest, slots[g].nnz);
-        // CTAs a graph: enough that the largest graph's share is a few steps each
-        const dim3 grid(g1 - g0, static_cast<unsigned>(std::min<int64_t>(std::max<int64_t>(largest >> 14, 8), 64)));
-        k_concat_graphs<<<grid, 256, 0, s>>>(dslots + g0, rp, col, key, bad);
-        k_set_last<<<1, 1, 0, s>>>(rp, v1, e1);  // the group's end (the next group writes the same value)
-        note_launches(2);
-        GK_CUDA(cudaGetLastError());
+        GK_CHECK(concat(g0, g1, v1, e1));
         // rows [v0, v1) against the whole combined matrix: their columns lie in
         // [v0, v1), so only this group's B rows are read
         DevCsr rows{v1 - v0, vtot, e1 - e0, rp + v0, col, nullptr};
@@ -694,8 +714,15 @@ int gk_tc_count_batched(const gk_csr *graphs, int ngraphs, uint64_t *counts, int
             GK_CHECK(tri_sample(in, check ? &f->chk : nullptr, &f->sample, s));
             GK_CUDA(cudaMemcpyAsync(&h, f, sizeof(Facts), cudaMemcpyDeviceToHost, s));
             GK_CUDA(cudaStreamSynchronize(s));
-            if (check) GK_CHECK(csr_verdict(rows, e0, v0, key, dranges, bad, CSR_SORTED, "graphs", h.chk, s, gs));
-            if (rows.nnz > 0) GK_CHECK(sched_prepare(sched, GK_ACCUM_AUTO));
+            // a defect comes before a mode that does not fit
+            const int verdict =
+                check ? csr_verdict(rows, e0, v0, key, dranges, bad, CSR_SORTED, "graphs", h.chk, s, gs) : GK_OK;
+            if (verdict == GK_ERR_INVALID_CSR) GK_CHECK(caller_defect());
+            GK_CHECK(verdict);
+            if (rows.nnz > 0 && sched_prepare(sched, GK_ACCUM_AUTO) != GK_OK) {
+                GK_CHECK(caller_defect());
+                return sched_prepare(sched, GK_ACCUM_AUTO);
+            }
             GK_CHECK(tri_count(in, h.chk, h.sample, d, s, &done));
         } else {
             cudaGetLastError();
