@@ -1541,6 +1541,23 @@ int tri_support(const DevCsr &L, TriSupport *out, cudaStream_t s, Scratch &scr, 
     return GK_OK;
 }
 
+// The graph in degree order, ready to be counted (nothing is added to the sums yet).
+static int degree_order(const TriInput &in, unsigned long long *sums, TriArgs *a, int *lb, cudaStream_t s,
+                        Scratch &scr) {
+    GK_CHECK(scr.reserve(static_cast<size_t>(tri_bytes(in.L.m, in.L.nnz))));
+    uint32_t *deg, *rank;
+    GK_CHECK(order_vertices(in, &deg, &rank, s, scr));
+    // Columns below the low limit are tested in the warp's bitmap, the others
+    // by filter and search.  2^15 keeps 40 warps an SM (2^16: 20, with 8 KB
+    // bitmaps): RMAT-22 count 3.3 against 3.9 ms; on RMAT-24, where more of the
+    // columns read lie beyond 2^15, 28.5 against 26.2 ms.
+    *lb = (in.key ? in.max_m : in.L.m) > (int64_t(1) << 23) ? 16 : 15;
+    GK_CHECK(orient(in, deg, rank, *lb, false, a, s, scr));
+    a->sums = sums;
+    a->key = in.key ? in.key + in.vbase : nullptr;
+    return GK_OK;
+}
+
 int tri_count(const TriInput &in, const CsrCheckOut &facts, unsigned long long sample, unsigned long long *sums,
               cudaStream_t s, bool *done) {
     *done = false;
@@ -1558,22 +1575,13 @@ int tri_count(const TriInput &in, const CsrCheckOut &facts, unsigned long long s
         return launch_walk(in, TriGate{}, facts.not_lower ? 0 : 1, sums, s);
     }
     if (facts.not_lower) return GK_OK;  // not a triangle: the sum depends on the order
-    // scratch beyond what the product needs: where memory is short, that runs
-    const int64_t bytes = tri_bytes(m, E);
-    if (!scratch_fits(bytes)) return GK_OK;
+    // scratch beyond what the product needs: where there is no room, that runs
     Scratch scr(s);
-    GK_CHECK(scr.reserve(static_cast<size_t>(bytes)));
-    uint32_t *deg, *rank;
-    GK_CHECK(order_vertices(in, &deg, &rank, s, scr));
-    // Columns below the low limit are tested in the warp's bitmap, the others
-    // by filter and search.  2^15 keeps 40 warps an SM (2^16: 20, with 8 KB
-    // bitmaps): RMAT-22 count 3.3 against 3.9 ms; on RMAT-24, where more of the
-    // columns read lie beyond 2^15, 28.5 against 26.2 ms.
-    const int lb = (in.key ? in.max_m : m) > (int64_t(1) << 23) ? 16 : 15;
     TriArgs a;
-    GK_CHECK(orient(in, deg, rank, lb, false, &a, s, scr));
-    a.sums = sums;
-    a.key = in.key ? in.key + in.vbase : nullptr;
+    int lb = 0;
+    const int status = degree_order(in, sums, &a, &lb, s, scr);
+    if (status == GK_ERR_OOM) return GK_OK;
+    GK_CHECK(status);
     if (lb == 16) GK_CHECK((in.key ? launch_count<16, true>(a, s) : launch_count<16, false>(a, s)));
     else GK_CHECK((in.key ? launch_count<15, true>(a, s) : launch_count<15, false>(a, s)));
     *done = true;
