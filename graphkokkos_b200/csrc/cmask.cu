@@ -529,8 +529,13 @@ extern "C" int gk_mxmm_cmask(const gk_csr *A, const gk_csr *B, const gk_csr *M, 
         // without room for the products (nothing is written before it is known) the windows serve
         Scratch own(s);
         const int status = cmask_by_sort(a, s, own);
-        if (status != GK_ERR_OOM) GK_CHECK(status);
-        done = status == GK_OK;
+        if (status == GK_ERR_OOM) {
+            own.release();
+            scratch_reclaim(s);
+        } else {
+            GK_CHECK(status);
+            done = true;
+        }
     }
     if (!done) GK_CHECK(fill ? launch_rows<true>(a, s) : launch_rows<false>(a, s));
     GK_CHECK(read_state());

@@ -116,22 +116,13 @@ void Scratch::release() {
     if (owned_) arena_ = nullptr;
 }
 
-bool scratch_fits(int64_t bytes) {
-    if (bytes < (int64_t(1) << 30)) return true;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
+void scratch_reclaim(cudaStream_t s) {
     int dev = 0;
     cudaMemPool_t pool;
-    uint64_t reserved = 0, used = 0;
+    cudaStreamSynchronize(s);
     cudaGetDevice(&dev);
-    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
-    }
-    return static_cast<double>(bytes) < 0.9 * (static_cast<double>(free_b) + static_cast<double>(reserved - used));
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    cudaGetLastError();
 }
 
 bool is_device_pointer(const void *p) {

@@ -139,10 +139,10 @@ int stage_csr(const gk_csr *in, DevCsr *out, Scratch &scr, cudaStream_t s, int64
 bool is_device_pointer(const void *p);
 int validate_csr_shape(const gk_csr *c, const char *name);
 
-// Whether that many more bytes of stream-ordered scratch are to be had (the
-// device's free memory and what its pool keeps).  Small requests are not asked
-// about: an allocation that fails then fails the call.
-bool scratch_fits(int64_t bytes);
+// After a failed allocation, before another path that needs less is tried: what
+// the pool holds and no one uses (the failed path's scratch, freed by then) goes
+// back to the device.  Waits for the stream.
+void scratch_reclaim(cudaStream_t s);
 
 // Device CSR transforms (abi.cu): the transpose (A.n + 1 row pointers out,
 // rows sorted; oval may be null) and the strict lower triangle.

@@ -70,7 +70,7 @@ int tri_sample(const TriInput &in, const CsrCheckOut *chk, unsigned long long *s
 // Support of every edge (the triangles it lies on) of the graph whose strict
 // lower triangle is L.  An edge's number is the place of its column in its row's
 // storage: unit * 8 + position in the unit (find it with tri_edge); rows keep
-// no hub class here.  false in *done: no room, or numbers beyond 32 bits.
+// no hub class here.  false in *done: numbers beyond 32 bits (no room: GK_ERR_OOM).
 struct TriSupport {
     TriGraph g;
     const uint32_t *rank = nullptr;  // of every vertex

@@ -473,59 +473,94 @@ __global__ void __launch_bounds__(256) k_peel_keep(PeelArgs a, int64_t cap, int3
 // it took 0.3 ms to build (RMAT-13, five passes: the call 0.78 -> 0.63 ms).
 constexpr int PEEL_AHEAD = 8;
 
-// k-truss of an undirected graph (rp, col: symmetric, sorted, no diagonal; row:
-// every entry's row); the truss is left in rp_res / col_res (scratch).  false in
-// *done: no room for it, nothing was done.
-static int ktruss_peel(int64_t m, int64_t nnz, const int64_t *rp, const int32_t *col, const int32_t *row, int k,
-                       int *iters_out, int64_t *nnz_out, int64_t **rp_res, int32_t **col_res, cudaStream_t s,
-                       Scratch &scr, bool *done) {
-    *done = false;
-    if (nnz >= (int64_t(1) << 32)) return GK_OK;
+// What the passes work on, and the truss's arrays (in scr, which outlives the call's
+// own scratch).
+struct PeelBuffers {
+    TriSupport ts;
+    PeelArgs a;
+    uint32_t *eid;
+    int32_t *keep;
+    int64_t *pos;
+    char *scan_tmp;
+    size_t scan_bytes;
+    int64_t *rp_res;
+    int32_t *col_res;
+    bool ok = false;
+};
+
+// The supports, and every allocation.
+static int peel_prepare(int64_t m, int64_t nnz, const int64_t *rp, const int32_t *col, const int32_t *row, int k,
+                        PeelBuffers *out, cudaStream_t s, Scratch &own, Scratch &scr) {
     const int sms = ctx().num_sms;
     const int64_t E = nnz / 2;
     int64_t *len, *lrp;
     int32_t *lcol;
+    size_t sb = 0, kb = 0;
+    GK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, sb, static_cast<int64_t *>(nullptr),
+                                          static_cast<int64_t *>(nullptr), m + 1, s));
+    GK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, kb, static_cast<int32_t *>(nullptr),
+                                          static_cast<int64_t *>(nullptr), nnz + 1, s));
+    out->scan_bytes = kb;
+    GK_CHECK(own.alloc(&out->scan_tmp, sb > kb ? sb : kb));
     Scratch low(s);  // the lower triangle, needed for the support only
     GK_CHECK(low.alloc(&len, m + 1));
     GK_CHECK(low.alloc(&lrp, m + 1));
     GK_CHECK(low.alloc(&lcol, E));
     GK_CUDA(cudaMemsetAsync(len + m, 0, sizeof(int64_t), s));
     k_lower_len<<<sms * 4, 256, 0, s>>>(m, rp, col, len);
-    size_t sb = 0, kb = 0;
-    GK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, sb, len, lrp, m + 1, s));
-    GK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, kb, static_cast<int32_t *>(nullptr),
-                                          static_cast<int64_t *>(nullptr), nnz + 1, s));
-    char *tmp;
-    GK_CHECK(scr.alloc(&tmp, sb > kb ? sb : kb));
-    GK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, sb, len, lrp, m + 1, s));
+    GK_CUDA(cub::DeviceScan::ExclusiveSum(out->scan_tmp, sb, len, lrp, m + 1, s));
     k_lower_fill<<<sms * 8, 256, 0, s>>>(m, rp, col, row, lrp, lcol);
     note_launches(2);
     GK_CUDA(cudaGetLastError());
-    TriSupport ts;
-    Scratch tri(s);
-    bool ok = false;
-    GK_CHECK(tri_support(DevCsr{m, m, E, lrp, lcol, nullptr}, &ts, s, tri, &ok));
-    if (!ok) return GK_OK;
+    GK_CHECK(tri_support(DevCsr{m, m, E, lrp, lcol, nullptr}, &out->ts, s, own, &out->ok));
+    if (!out->ok) return GK_OK;
     low.release();
-    PeelArgs a;
+    PeelArgs &a = out->a;
     a.m = m;
     a.rp = rp;
     a.col = col;
     a.row = row;
-    a.sup = ts.sup;
+    a.sup = out->ts.sup;
     a.thresh = k - 2;
-    uint32_t *eid;
-    int32_t *keep;
-    int64_t *pos;
-    GK_CHECK(scr.alloc(&eid, nnz));
-    GK_CHECK(scr.alloc(&a.mark, ts.numbers));
-    GK_CHECK(scr.alloc(&a.list[0], E));
-    GK_CHECK(scr.alloc(&a.list[1], E));
-    GK_CHECK(scr.alloc(&a.st, 1));
-    GK_CHECK(scr.alloc(&keep, nnz + 1));
-    GK_CHECK(scr.alloc(&pos, nnz + 1));
-    GK_CHECK(scr.alloc(rp_res, m + 1));
-    GK_CHECK(scr.alloc(col_res, nnz));
+    GK_CHECK(own.alloc(&out->eid, nnz));
+    GK_CHECK(own.alloc(&a.mark, out->ts.numbers));
+    GK_CHECK(own.alloc(&a.list[0], E));
+    GK_CHECK(own.alloc(&a.list[1], E));
+    GK_CHECK(own.alloc(&a.st, 1));
+    GK_CHECK(own.alloc(&out->keep, nnz + 1));
+    GK_CHECK(own.alloc(&out->pos, nnz + 1));
+    GK_CHECK(scr.alloc(&out->rp_res, m + 1));
+    return scr.alloc(&out->col_res, nnz);
+}
+
+// k-truss of an undirected graph (rp, col: symmetric, sorted, no diagonal; row:
+// every entry's row); the truss is left in rp_res / col_res (scratch).  false in
+// *done: no room for it, and what it took has been given back.
+static int ktruss_peel(int64_t m, int64_t nnz, const int64_t *rp, const int32_t *col, const int32_t *row, int k,
+                       int *iters_out, int64_t *nnz_out, int64_t **rp_res, int32_t **col_res, cudaStream_t s,
+                       Scratch &scr, bool *done) {
+    *done = false;
+    if (nnz >= (int64_t(1) << 32)) return GK_OK;
+    const int sms = ctx().num_sms;
+    Scratch own(s);
+    PeelBuffers b;
+    const int status = peel_prepare(m, nnz, rp, col, row, k, &b, s, own, scr);
+    if (status == GK_ERR_OOM) {
+        own.release();
+        scratch_reclaim(s);
+        return GK_OK;
+    }
+    GK_CHECK(status);
+    if (!b.ok) return GK_OK;
+    PeelArgs &a = b.a;
+    const TriSupport &ts = b.ts;
+    uint32_t *eid = b.eid;
+    int32_t *keep = b.keep;
+    int64_t *pos = b.pos;
+    char *tmp = b.scan_tmp;
+    size_t kb = b.scan_bytes;
+    *rp_res = b.rp_res;
+    *col_res = b.col_res;
     a.eid = eid;
     GK_CUDA(cudaMemsetAsync(a.mark, 0, sizeof(uint32_t) * ts.numbers, s));
     PeelState init{};

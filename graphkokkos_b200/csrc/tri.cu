@@ -1518,9 +1518,7 @@ int tri_support(const DevCsr &L, TriSupport *out, cudaStream_t s, Scratch &scr, 
     const int64_t m = L.m, E = L.nnz;
     out->numbers = 8 * (E / 4 + 2 * std::min(m, E) + 2);
     if (m < 2 || E < 1 || out->numbers >= (int64_t(1) << 32)) return GK_OK;
-    const int64_t bytes = tri_bytes(m, E) + 4 * out->numbers;
-    if (!scratch_fits(bytes)) return GK_OK;
-    GK_CHECK(scr.reserve(static_cast<size_t>(bytes)));
+    GK_CHECK(scr.reserve(static_cast<size_t>(tri_bytes(m, E) + 4 * out->numbers)));
     TriInput in;
     in.L = L;
     uint32_t *deg, *rank;
@@ -1580,7 +1578,11 @@ int tri_count(const TriInput &in, const CsrCheckOut &facts, unsigned long long s
     TriArgs a;
     int lb = 0;
     const int status = degree_order(in, sums, &a, &lb, s, scr);
-    if (status == GK_ERR_OOM) return GK_OK;
+    if (status == GK_ERR_OOM) {
+        scr.release();
+        scratch_reclaim(s);
+        return GK_OK;
+    }
     GK_CHECK(status);
     if (lb == 16) GK_CHECK((in.key ? launch_count<16, true>(a, s) : launch_count<16, false>(a, s)));
     else GK_CHECK((in.key ? launch_count<15, true>(a, s) : launch_count<15, false>(a, s)));

@@ -44,3 +44,20 @@ def test_batch_without_room_for_the_degree_order(gk, orc, cuda):
     want = np.array([orc.tc_lower(x) for x in host], dtype=np.uint64)
     failed = failures(gk, lambda: gk.tc_count_batched(graphs), lambda got: np.testing.assert_array_equal(got, want), 60)
     assert len(failed) <= 12, failed  # the combined matrix, the tables and a word per group
+
+
+def test_ktruss_without_room_for_the_peeling(gk, orc, cuda):
+    """The product loop takes over, whichever of the peeling's allocations fails."""
+    A = gk.gen_rmat(11, 16, seed=6)
+    rp, col, iters, _ = orc.ktruss(A, 5)
+    G = A.to("cuda")
+
+    def same(got):
+        T, it = got
+        assert it == iters
+        np.testing.assert_array_equal(T.rowptr.cpu().numpy(), rp)
+        np.testing.assert_array_equal(T.col.cpu().numpy(), col)
+
+    failed = failures(gk, lambda: gk.ktruss(G, 5), same, 60)
+    # the matrix's copies, the check's word, the entries' rows and the symmetry's counters
+    assert failed == list(range(5)), failed
