@@ -61,3 +61,17 @@ def test_ktruss_without_room_for_the_peeling(gk, orc, cuda):
     failed = failures(gk, lambda: gk.ktruss(G, 5), same, 60)
     # the matrix's copies, the check's word, the entries' rows and the symmetry's counters
     assert failed == list(range(5)), failed
+
+
+@pytest.mark.parametrize("nsrc", [100, 600])
+def test_bc_without_room_for_a_wide_chunk(gk, orc, cuda, nsrc):
+    """A chunk whose allocations fail is narrowed; one of 32 sources needs them all
+    (one reservation and the eight arrays carved from it)."""
+    from tests import graphs as G
+    A = gk.gen_rmat(11, 8, seed=6)
+    src = np.random.default_rng(1).permutation(A.m)[:nsrc]
+    want, want20 = orc.bc_f64(A, src), orc.bc_f64(A, src[:20])
+    D = A.to("cuda")
+    wide = failures(gk, lambda: gk.bc_batch(D, src).cpu().numpy(), lambda got: G.assert_bc_close(got, want), 60)
+    narrow = failures(gk, lambda: gk.bc_batch(D, src[:20]).cpu().numpy(), lambda got: G.assert_bc_close(got, want20), 60)
+    assert len(wide) == len(narrow) - 9, (wide, narrow)
