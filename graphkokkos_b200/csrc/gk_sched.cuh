@@ -49,7 +49,8 @@ struct Variant {
     int comp;       // block HASH kinds: filter candidates packed into a per-warp queue and checked one per lane
 };
 
-constexpr int NV = 24;
+constexpr int NV = 24;      // the catalogue: the model's outputs, variants that can be forced
+constexpr int NK = NV + 2;  // kernels of the engine
 // Shared-memory budget of every variant is below 160 KB; see the kernels.
 // Tables are bucketed (four slots per 16-byte load).  The small ones run at
 // load factor <= 1/4 (chunk <= cap/4); the large ones of variants 6-8 and
@@ -57,9 +58,11 @@ constexpr int NV = 24;
 // entry) send only filter candidates to the table; variants 12-14 have none
 // and look every streamed element up in the table directly, which wins on
 // rows where a large share of the elements are mask columns.
-// Variants 1 and 2 (K_PACKED_CTA, K_PACKED) pack the elements of 32 B rows at a
-// time onto the lanes and look mask candidates up in the sorted mask row; most of
-// their rows come from the row rule of spgemm.cu, not from a bin.
+// The two kernels behind the catalogue (NV, NV + 1: K_PACKED_CTA, K_PACKED) pack the
+// elements of 32 B rows at a time onto the lanes and look mask candidates up in the
+// sorted mask row.  Their rows come from the row rule of spgemm.cu and the plain
+// heuristic; they are no outputs of the model and cannot be forced, so that models
+// and variant numbers saved with the 24 variants keep their meaning.
 // Variant 17 (K_SEARCH) does not stream B rows: a warp per row looks each mask
 // column inside B_k's column range up in B_k by binary search (mask chunks of
 // 256 columns in shared memory), which wins where mask rows are short and B
@@ -79,8 +82,8 @@ constexpr int NV = 24;
 // one to one, so a hit there needs no table lookup when only sums are kept)
 #define GK_VARIANT_TABLE { \
     {K_HASH_GROUP,   4,  4,    64,    64,    16,    16,   0,  0, 1, 3  , 0, 0},   \
-    {K_PACKED_CTA, 128, 32,  1024,  1024,  1024,  1024,   0, 15, 1, 3  , 0, 0},   \
-    {K_PACKED,      32, 32,   256,   256,   256,   256,   0, 13, 1, 3  , 0, 0},   \
+    {K_HASH_GROUP,   8,  8,   128,   128,    32,    32,   0,  0, 1, 3  , 0, 0},   \
+    {K_HASH_GROUP,  32, 32,   512,   512,   128,   128,   0, 13, 1, 3  , 0, 0},   \
     {K_HASH_BLOCK,  64, 32,   512,   512,   128,   128,  16, 13, 8, 3  , 0, 0},   \
     {K_HASH_BLOCK, 128, 32,  1024,  1024,   256,   256,  17, 14, 4, 3  , 0, 0},   \
     {K_HASH_BLOCK, 128, 16,  1024,  1024,   256,   256,  17, 14, 4, 3  , 0, 0},   \
@@ -102,15 +105,17 @@ constexpr int NV = 24;
     {K_HASH_BLOCK, 512, 32,  8192, 16384,  4096,  8192,  20, 16, 1, 3  , 18, 1}, \
     {K_SEARCH,      16, 16,    64,    64,    64,    64,   0,  0, 2, 0  , 0, 0},   \
     {K_SEARCH,       8,  8,    32,    32,    32,    32,   0,  0, 2, 0  , 0, 0},   \
+    {K_PACKED_CTA, 128, 32,  1024,  1024,  1024,  1024,   0, 15, 1, 3  , 0, 0},   \
+    {K_PACKED,      32, 32,   256,   256,   256,   256,   0, 13, 1, 3  , 0, 0},   \
 }
-constexpr Variant VARIANTS[NV] = GK_VARIANT_TABLE;
+constexpr Variant VARIANTS[NK] = GK_VARIANT_TABLE;
 #ifdef __CUDACC__
-__constant__ const Variant c_variants[NV] = GK_VARIANT_TABLE;  // runtime-indexed copy for device code
+__constant__ const Variant c_variants[NK] = GK_VARIANT_TABLE;  // runtime-indexed copy for device code
 #endif
 constexpr int NT_GROUP = 256;  // CTA size of the group kinds
 __host__ __device__ constexpr int group_cta_threads(int) { return NT_GROUP; }
 // variant ids the heuristics name
-constexpr int V_PACKED_CTA = 1, V_PACKED = 2, V_MCA_GROUP = 9, V_MCA_BLOCK = 10, V_MSA_BLOCK = 11;
+constexpr int V_PACKED_CTA = NV, V_PACKED = NV + 1, V_MCA_GROUP = 9, V_MCA_BLOCK = 10, V_MSA_BLOCK = 11;
 
 // Variants the learned scheduler (and the autotuner) may pick for a bin: a
 // variant is excluded where it would split every mask row into many chunks

@@ -18,7 +18,7 @@
 //                   get their item count (mask chunks x A-entry splits)
 //  5. one persistent kernel per variant over its rows / items (the catalogue
 //     of 24 variants is the table in gk_sched.cuh):
-//       HASH_GROUP  4 threads per row, the mask row's columns in a
+//       HASH_GROUP  4, 8 or 32 threads per row, the mask row's columns in a
 //                   shared-memory bucketed hash set (slot = accumulator)
 //       PACKED      a warp or a CTA per row, B elements packed onto the lanes,
 //                   sorted mask row behind a filter (gk_kpacked.cuh)
@@ -303,8 +303,8 @@ __device__ __forceinline__ int64_t row_items(const DevCsr &A, const DevCsr &M, c
 __global__ void k_count_rows(DevCsr A, DevCsr M, const int64_t *work, const uint16_t *bin, const int *var_of_bin,
                              int force_variant, bool write, int *vcount, int *vsimple, Gate gate) {
     if (!gate.open()) return;
-    __shared__ int s_cnt[NV], s_simple[NV];
-    if (threadIdx.x < NV) s_cnt[threadIdx.x] = s_simple[threadIdx.x] = 0;
+    __shared__ int s_cnt[NK], s_simple[NK];
+    if (threadIdx.x < NK) s_cnt[threadIdx.x] = s_simple[threadIdx.x] = 0;
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < A.m; r += stride) {
@@ -314,7 +314,7 @@ __global__ void k_count_rows(DevCsr A, DevCsr M, const int64_t *work, const uint
         if (row_items(A, M, work, r, v, write) == 1) atomicAdd(&s_simple[v], 1);
     }
     __syncthreads();
-    if (threadIdx.x < NV && s_cnt[threadIdx.x]) {
+    if (threadIdx.x < NK && s_cnt[threadIdx.x]) {
         atomicAdd(&vcount[threadIdx.x], s_cnt[threadIdx.x]);
         atomicAdd(&vsimple[threadIdx.x], s_simple[threadIdx.x]);
     }
@@ -324,14 +324,14 @@ __global__ void k_count_rows(DevCsr A, DevCsr M, const int64_t *work, const uint
 __global__ void k_offsets(const int *vcount, const int *vsimple, int *voff, int *vcursor, unsigned int *fetch) {
     if (threadIdx.x == 0) {
         int acc = 0;
-        for (int v = 0; v < NV; ++v) {
+        for (int v = 0; v < NK; ++v) {
             voff[v] = acc;
             vcursor[2 * v] = acc;
             vcursor[2 * v + 1] = acc + vsimple[v];
             fetch[v] = 0;
             acc += vcount[v];
         }
-        voff[NV] = acc;
+        voff[NK] = acc;
     }
 }
 
@@ -339,10 +339,10 @@ __global__ void k_scatter_rows(DevCsr A, DevCsr M, const int64_t *work, const ui
                                const int *var_of_bin, int force_variant, bool write, int *vcursor,
                                int32_t *rowlist, int64_t *item_n, Gate gate) {
     if (!gate.open()) return;
-    __shared__ int s_cnt[2 * NV], s_base[2 * NV];
+    __shared__ int s_cnt[2 * NK], s_base[2 * NK];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < A.m; base += stride) {
-        if (threadIdx.x < 2 * NV) s_cnt[threadIdx.x] = 0;
+        if (threadIdx.x < 2 * NK) s_cnt[threadIdx.x] = 0;
         __syncthreads();
         const int64_t r = base + threadIdx.x;
         int slot = -1, local = 0;
@@ -356,7 +356,7 @@ __global__ void k_scatter_rows(DevCsr A, DevCsr M, const int64_t *work, const ui
             }
         }
         __syncthreads();
-        if (threadIdx.x < 2 * NV && s_cnt[threadIdx.x])
+        if (threadIdx.x < 2 * NK && s_cnt[threadIdx.x])
             s_base[threadIdx.x] = atomicAdd(&vcursor[threadIdx.x], s_cnt[threadIdx.x]);
         __syncthreads();
         if (slot >= 0) {
@@ -639,10 +639,10 @@ __device__ __forceinline__ BRow brow_of(const KArgs &p, int k, int64_t t) {
 // Streams the B rows of A entries t = first, first+step, ... < a1 with one
 // sub-group of SUB lanes: the next entry's row bounds and the entry after
 // that's column are loaded while the current row streams.
-template <int SUB, int CAP, int PK, bool ACC, bool VAL>
+template <int SUB, int CAP, int PK, bool ACC, bool VAL, int FLOG>
 __device__ __forceinline__ void stream_entries(const KArgs &p, int64_t first, int64_t a1, int step, int sl,
                                                bool chunked, int lo_col, int hi_col, const int *keys, int *acc,
-                                               int clen, unsigned &cnt) {
+                                               int clen, unsigned &cnt, const unsigned *filt) {
     const unsigned smask = group_mask<SUB>();
     int64_t t = first;
     if (t >= a1) return;
@@ -664,7 +664,8 @@ __device__ __forceinline__ void stream_entries(const KArgs &p, int64_t first, in
                 }
             }
             if (!skip)
-                stream_row<SUB, CAP, PK, ACC, VAL>(p, cur.b0, cur.b1, sl, cur.av, keys, acc, clen, cnt, nullptr, hi_col);
+                stream_row<SUB, CAP, PK, ACC, VAL, FLOG>(p, cur.b0, cur.b1, sl, cur.av, keys, acc, clen, cnt, filt,
+                                                         hi_col);
         }
         t = tn;
     }
@@ -679,11 +680,12 @@ __host__ __device__ constexpr int c_group_fetch() { return G >= 32 ? 2 : 4; }
 // sub-groups of SUB lanes that stream their B rows concurrently.  Each group
 // takes its next row from a global counter, so groups never wait on each
 // other for work.
-template <int G, int SUB, int NT, int CAP, int CHUNK, bool MCA, int EPI, bool VAL>
+template <int G, int SUB, int NT, int CAP, int CHUNK, bool MCA, int FLOG, int EPI, bool VAL>
 __global__ void __launch_bounds__(NT, GK_LB_THREADS / NT) k_group(KArgs p) {
     constexpr int NG = NT / G;
     constexpr int S = G / SUB;
     constexpr bool ACC = (EPI == EPI_WRITE);
+    constexpr int FW = (!MCA && FLOG > 0) ? (1 << FLOG) / 32 : 0;  // filter words per group
     extern __shared__ int smem[];
     const int g = threadIdx.x / G;
     const int lane = threadIdx.x % G;
@@ -694,6 +696,7 @@ __global__ void __launch_bounds__(NT, GK_LB_THREADS / NT) k_group(KArgs p) {
     int *const keys0 = smem + g * KST;
     int *keys = keys0;
     int *acc = smem + NG * KST + g * CAP;
+    unsigned *filt = reinterpret_cast<unsigned *>(smem + NG * KST + NG * CAP * (ACC ? 1 : 0)) + g * FW;
     const unsigned gmask = group_mask<G>();
     const int begin = p.voff[p.v], end = p.voff[p.v + 1];
     unsigned long long local = 0;
@@ -701,12 +704,13 @@ __global__ void __launch_bounds__(NT, GK_LB_THREADS / NT) k_group(KArgs p) {
     // graph of a batch), so a group adds up per key and flushes on change
     int cur_key = -1;
     unsigned long long cur_sum = 0;
-    // the table starts empty; every row clears what it set
+    // the table and filter start empty; every row clears what it set
     if constexpr (!MCA) {
         for (int s = lane; s < CAP; s += G) {
             keys[s] = EMPTY_KEY;
             if (ACC) acc[s] = 0;
         }
+        for (int wd = lane; wd < FW; wd += G) filt[wd] = 0u;
     }
     __syncwarp(gmask);
     constexpr int FB = c_group_fetch<G>();
@@ -738,21 +742,28 @@ __global__ void __launch_bounds__(NT, GK_LB_THREADS / NT) k_group(KArgs p) {
                     for (int q = lane; q < clen; q += G) acc[q] = 0;
                 cp_async_wait_all();
             } else {
-                for (int q = c0 + lane; q < c1; q += G) hash_insert<CAP>(keys, mc[q]);
+                for (int q = c0 + lane; q < c1; q += G) {
+                    const int x = mc[q];
+                    hash_insert<CAP>(keys, x);
+                    if constexpr (FW > 0) {
+                        const uint32_t h = filter_bit<FLOG>(x);
+                        atomicOr(filt + (h >> 5), 1u << (h & 31));
+                    }
+                }
             }
             __syncwarp(gmask);
             const int lo_col = mc[c0], hi_col = mc[c1 - 1];
             unsigned cnt = 0;
-            stream_entries<SUB, CAP, MCA ? PK_MCA : PK_HASH, ACC, VAL>(p, a0 + sg, a1, S, sl, chunked, lo_col, hi_col,
-                                                                      keys, acc, clen, cnt);
+            stream_entries<SUB, CAP, MCA ? PK_MCA : PK_HASH, ACC, VAL, (FW > 0 ? FLOG : 0)>(
+                p, a0 + sg, a1, S, sl, chunked, lo_col, hi_col, keys, acc, clen, cnt, filt);
             __syncwarp(gmask);
             if constexpr (MCA) {
                 if (ACC)
                     for (int q = c0 + lane; q < c1; q += G) p.c_val[m0 + q] = acc[q - c0];
             } else {
                 // find this chunk's slots (writing the values out), then clear
-                // them only after every lane has found its keys, so that no
-                // probe meets a half-cleared bucket
+                // them and the filter words only after every lane has found
+                // its keys, so that no probe meets a half-cleared bucket
                 constexpr int PER = (CHUNK + G - 1) / G;
                 int slot[PER];
 #pragma unroll
@@ -763,11 +774,16 @@ __global__ void __launch_bounds__(NT, GK_LB_THREADS / NT) k_group(KArgs p) {
                 }
                 __syncwarp(gmask);
 #pragma unroll
-                for (int k = 0; k < PER; ++k)
+                for (int k = 0; k < PER; ++k) {
+                    const int q = c0 + lane + k * G;
                     if (slot[k] >= 0) {
                         keys[slot[k]] = EMPTY_KEY;
                         if (ACC) acc[slot[k]] = 0;
                     }
+                    if constexpr (FW > 0) {
+                        if (q < c1) filt[filter_bit<FLOG>(mc[q]) >> 5] = 0u;
+                    }
+                }
             }
             if (!ACC) rowsum += cnt;
             __syncwarp(gmask);
@@ -809,8 +825,9 @@ constexpr size_t smem_bytes(bool write) {
         const int nt = group_cta_threads(V);
         const int ng = nt / X.G;
         const int cap = (X.kind == K_MCA_GROUP) ? X.chunk : X.cap;
+        const size_t filter = (X.kind == K_HASH_GROUP && X.flog > 0) ? (size_t(1) << X.flog) / 8 : 0;
         const size_t stage_pad = (X.kind == K_MCA_GROUP) ? 16 : 0;  // cp.async alignment slots
-        return size_t(ng) * (size_t(cap) * 4 * (write ? 2 : 1) + stage_pad);
+        return size_t(ng) * (size_t(cap) * 4 * (write ? 2 : 1) + filter + stage_pad);
     } else if constexpr (X.kind == K_PACKED) {
         return size_t(NT_GROUP / 32) * (size_t(X.cap) * 4 * (write ? 2 : 1) + (size_t(1) << X.flog) / 8);
     } else if constexpr (X.kind == K_PACKED_CTA) {
@@ -843,7 +860,7 @@ static cudaError_t launch_variant_t(const KArgs &args, int num_sms, cudaStream_t
         constexpr int NTV = group_cta_threads(V);
         constexpr bool MCA = X.kind == K_MCA_GROUP;
         constexpr int CAPV = MCA ? X.chunk : X.cap;
-        fn = k_group<X.G, X.sub, NTV, CAPV, X.chunk, MCA, EPI, VAL>;
+        fn = k_group<X.G, X.sub, NTV, CAPV, X.chunk, MCA, (MCA ? 0 : X.flog), EPI, VAL>;
         nt = NTV;
     } else if constexpr (X.kind == K_PACKED) {
         fn = k_packed<X.cap, X.flog, EPI, VAL>;
@@ -915,13 +932,15 @@ static cudaError_t launch_variant(int v, const KArgs &a, int epi, bool val, int 
         case 21: return launch_variant_v<21>(a, epi, val, sms, s, launch);
         case 22: return launch_variant_v<22>(a, epi, val, sms, s, launch);
         case 23: return launch_variant_v<23>(a, epi, val, sms, s, launch);
+        case V_PACKED_CTA: return launch_variant_v<V_PACKED_CTA>(a, epi, val, sms, s, launch);
+        case V_PACKED: return launch_variant_v<V_PACKED>(a, epi, val, sms, s, launch);
         default: return cudaErrorInvalidValue;
     }
 }
 
 int spgemm_prepare(int epi, bool values, int sched, int force_accum) {
     KArgs none{};
-    for (int v = 0; v < NV; ++v) {
+    for (int v = 0; v < NK; ++v) {
         cudaError_t e = launch_variant(v, none, epi, values, ctx().num_sms, nullptr, false);
         if (e != cudaSuccess) return cuda_fail(e, "masked SpGEMM variant setup");
     }
@@ -934,15 +953,16 @@ size_t spgemm_scratch_bytes(int64_t m) {
     cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, static_cast<int64_t *>(nullptr),
                                   static_cast<int64_t *>(nullptr), m + 1);
     return r(8 * m) + r(4 * m) + r(2 * m) + r(4 * m) + 2 * r(8 * (m + 1)) + r(sizeof(BinStats) * NBINS) +
-           r(4 * NBINS) + r(4 * (6 * NV + 4)) + r(4 * NV) + r(tmp_bytes);
+           r(4 * NBINS) + r(4 * (6 * NK + 4)) + r(4 * NK) + r(tmp_bytes);
 }
 
 // NVTX range names of the variant launches
-static const char *const kVariantRange[NV] = {
+static const char *const kVariantRange[NK] = {
     "gk:variant 0",  "gk:variant 1",  "gk:variant 2",  "gk:variant 3",  "gk:variant 4",  "gk:variant 5",
     "gk:variant 6",  "gk:variant 7",  "gk:variant 8",  "gk:variant 9",  "gk:variant 10", "gk:variant 11",
     "gk:variant 12", "gk:variant 13", "gk:variant 14", "gk:variant 15", "gk:variant 16", "gk:variant 17",
-    "gk:variant 18", "gk:variant 19", "gk:variant 20", "gk:variant 21", "gk:variant 22", "gk:variant 23"};
+    "gk:variant 18", "gk:variant 19", "gk:variant 20", "gk:variant 21", "gk:variant 22", "gk:variant 23",
+    "gk:packed CTA", "gk:packed"};
 
 // ---------------------------------------------------------------------------
 // driver
@@ -987,13 +1007,13 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     GK_CHECK(scr.alloc(&item_ex, m + 1));
     GK_CHECK(scr.alloc(&bins, NBINS));
     GK_CHECK(scr.alloc(&var_of_bin, NBINS));
-    GK_CHECK(scr.alloc(&vcount, 6 * NV + 4));
-    voff = vcount + NV;
-    vcursor = voff + NV + 1;          // 2 * NV
-    int *vsimple = vcursor + 2 * NV;  // NV
-    GK_CHECK(scr.alloc(&fetch, NV));
+    GK_CHECK(scr.alloc(&vcount, 6 * NK + 4));
+    voff = vcount + NK;
+    vcursor = voff + NK + 1;          // 2 * NK
+    int *vsimple = vcursor + 2 * NK;  // NK
+    GK_CHECK(scr.alloc(&fetch, NK));
     GK_CUDA(cudaMemsetAsync(bins, 0, sizeof(BinStats) * NBINS, s));
-    GK_CUDA(cudaMemsetAsync(vcount, 0, sizeof(int) * (6 * NV + 4), s));
+    GK_CUDA(cudaMemsetAsync(vcount, 0, sizeof(int) * (6 * NK + 4), s));
     GK_CUDA(cudaMemsetAsync(item_n, 0, sizeof(int64_t) * (m + 1), s));
 
     const int sms = c.num_sms;
@@ -1045,7 +1065,7 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     // that only those are launched (an empty persistent grid costs 2 to 10 us,
     // and there are 24).  Inside a capture, or with the checks switched off (the
     // call is then asynchronous), all of them are.
-    int hoff[NV + 1];
+    int hoff[NK + 1];
     bool known = false;
     if (csr_check_active(s)) {
         GK_CUDA(cudaMemcpyAsync(hoff, voff, sizeof(hoff), cudaMemcpyDeviceToHost, s));
@@ -1080,18 +1100,20 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
         const char *e = getenv("GK_CONCURRENT_VARIANTS");
         return e && e[0] == '1';
     }();
-    static_assert(NV <= kSideStreams, "one side stream per variant");
+    static_assert(NK <= kSideStreams, "one side stream per kernel");
     SideStreams &side = side_streams();
     const bool fork = concurrent && rq.force_variant < 0;
     if (fork) GK_CUDA(cudaEventRecord(side.fork, s));
-    ProfWindow prof(s, NV);
-    cudaEvent_t tev[NV + 1];
+    // the profile's numbers NV and NV + 1 are the triangle count's kernels (tri.cu)
+    auto slot = [](int v) { return v < NV ? v : v + 2; };
+    ProfWindow prof(s, NK + 2);
+    cudaEvent_t tev[NK + 1];
     const bool timed = rq.variant_ms_out != nullptr;
     if (timed) {
-        for (int v = 0; v <= NV; ++v) GK_CUDA(cudaEventCreate(&tev[v]));
+        for (int v = 0; v <= NK; ++v) GK_CUDA(cudaEventCreate(&tev[v]));
         GK_CUDA(cudaEventRecord(tev[0], s));
     }
-    for (int v = 0; v < NV; ++v) {
+    for (int v = 0; v < NK; ++v) {
         if ((rq.force_variant >= 0 && v != rq.force_variant) || (known && hoff[v] == hoff[v + 1])) {
             if (timed) GK_CUDA(cudaEventRecord(tev[v + 1], s));
             continue;
@@ -1103,10 +1125,10 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
             GK_CUDA(cudaStreamWaitEvent(vs, side.fork, 0));
         }
         NvtxRange vrange(kVariantRange[v]);
-        prof.begin(v, vs);
+        prof.begin(slot(v), vs);
         cudaError_t e = launch_variant(v, args, rq.epi, val, sms, vs);
         if (e != cudaSuccess) return cuda_fail(e, "masked SpGEMM variant launch");
-        prof.end(v, vs);
+        prof.end(slot(v), vs);
         note_launches(1);
         if (fork) {
             GK_CUDA(cudaEventRecord(side.join[v], vs));
@@ -1115,13 +1137,13 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
         if (timed) GK_CUDA(cudaEventRecord(tev[v + 1], s));
     }
     if (timed) {
-        GK_CUDA(cudaEventSynchronize(tev[NV]));
+        GK_CUDA(cudaEventSynchronize(tev[NK]));
         for (int v = 0; v < NV; ++v) {
             float ms = 0.f;
             GK_CUDA(cudaEventElapsedTime(&ms, tev[v], tev[v + 1]));
             rq.variant_ms_out[v] = ms;
         }
-        for (int v = 0; v <= NV; ++v) cudaEventDestroy(tev[v]);
+        for (int v = 0; v <= NK; ++v) cudaEventDestroy(tev[v]);
     }
     if (prof.active()) {
         // attribute the bins' work to the variants that ran them
@@ -1130,16 +1152,20 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
         GK_CUDA(cudaMemcpyAsync(hb, bins, sizeof(hb), cudaMemcpyDeviceToHost, s));
         GK_CUDA(cudaMemcpyAsync(hv, var_of_bin, sizeof(hv), cudaMemcpyDeviceToHost, s));
         GK_CUDA(cudaStreamSynchronize(s));
-        ProfTotals tot[NV] = {};
+        ProfTotals tot[NK + 2] = {};
         for (int b = 0; b < NBINS; ++b) {
             if (!hb[b].rows) continue;
             const int v = rq.force_variant >= 0 ? rq.force_variant : (rq.bin_variant ? rq.bin_variant[b] : hv[b]);
-            if (v < 0 || v >= NV) continue;
-            tot[v].rows += hb[b].rows;
-            tot[v].sum_a += hb[b].sum_a;
-            tot[v].sum_m += hb[b].sum_m;
-            tot[v].sum_work += hb[b].sum_work;
+            if (v < 0 || v >= NK) continue;
+            ProfTotals &t = tot[slot(v)];
+            t.rows += hb[b].rows;
+            t.sum_a += hb[b].sum_a;
+            t.sum_m += hb[b].sum_m;
+            t.sum_work += hb[b].sum_work;
         }
+        // the rows that the row rule took are in no bin: their number alone is known
+        if (known)
+            for (int v = NV; v < NK; ++v) tot[slot(v)].rows = hoff[v + 1] - hoff[v];
         GK_CHECK(prof.finish(tot));
     }
     return GK_OK;

@@ -373,9 +373,11 @@ int gk_bc_tune(const gk_csr *A, const int32_t *sources, int nsources, int shape,
 /* One record per kernel-variant launch of a masked SpGEMM call made while
  * profiling is on: CUDA-event time of the launch and the rows / A entries /
  * mask entries / streamed B entries (work) it processed.
- * Two further numbers stand for the triangle count's own kernels:
- * gk_sched_num_variants() the degree-ordered count (work: 16-byte units of
- * columns read), the next one the kernels without a plan (work 0).
+ * Further numbers, from gk_sched_num_variants() on: the degree-ordered triangle
+ * count (work: 16-byte units of columns read), the count's kernels without a plan
+ * (work 0), and the two packed kinds that rows with few products go to whatever
+ * the schedule (a CTA and a warp a row; of the rows that no bin holds, only their
+ * number).
  * Mode 1 synchronises the stream after each call and fills the work fields;
  * mode 2 only brackets the launches with events (no synchronisation, work
  * fields 0) and gk_prof_flush() resolves them; mode 0 turns profiling off. */
