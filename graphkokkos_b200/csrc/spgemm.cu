@@ -90,15 +90,27 @@ struct Gate {
 // learned schedule, m x k x n (A, B, M entries a row):
 //   20,011 x 15,013 x 18,013 (24, 40, 48)   282 / 239
 //   50,000 x 50,000 x 50,000 (40, 60, 60)   787 / 562
-//   Erdos-Renyi 20,000 (30) on itself        278 / 159; RMAT-12 LLL 296 / 303
-// and plain: 708 / 250, 1631 / 560, 840 / 158, 1580 / 933.
+//   Erdos-Renyi 20,000 (30) on itself        278 / 159
+// and plain: 708 / 250, 1631 / 560, 840 / 158; RMAT-12 L·L under L 2000 / 1430.
 constexpr int64_t PACKED_WORK = 2048, PACKED_DENSE_WORK = 512;
 constexpr int64_t PACKED_CTA_WORK = 1 << 16, PACKED_CTA_MEAN = 128;
 constexpr int64_t PACKED_SHARE = 20;
 
-enum : int { PACK_NONE = 0, PACK_WARP = 1, PACK_CTA = 2 };
-__device__ __forceinline__ uint16_t packed_bin(int pack, int64_t mlen, int64_t alen, int64_t work, int64_t n) {
+// The model knows good variants for sums (nothing to write back), most of all for
+// rows of a handful of products and for skewed rows: with it, sums take the rule only
+// where rows have PACKED_FLAT_MEAN products on average, and only rows whose longest B
+// row has PACKED_FLAT_B columns.  us, row sums and L·U count, learned, all rows by
+// the rule / none: Erdos-Renyi 1,000,000 (8) 769, 1398 / 527, 1185; 300,000 (24) 383,
+// 760 / 491, 1007; 20,000 (30) 149, 283 / 266, 365; RMAT-20 row sums, all / flat rows /
+// none: 8959 / 8826 / 8824.
+constexpr double PACKED_FLAT_MEAN = 64.0;
+constexpr int64_t PACKED_FLAT_B = 64;
+
+enum : int { PACK_NONE = 0, PACK_FLAT = 1, PACK_WARP = 2, PACK_CTA = 3 };
+__device__ __forceinline__ uint16_t packed_bin(int pack, int64_t mlen, int64_t alen, int64_t work, int64_t maxb,
+                                               int64_t n) {
     const bool sparse = mlen * PACKED_SHARE <= n;
+    if (pack == PACK_FLAT && maxb > PACKED_FLAT_B) return BIN_SKIP;
     if (work <= (sparse ? PACKED_WORK : PACKED_DENSE_WORK) && mlen <= VARIANTS[V_PACKED].cap) return BIN_PACKED;
     if (pack == PACK_CTA && sparse && work <= PACKED_CTA_WORK && work <= PACKED_CTA_MEAN * alen &&
         mlen <= VARIANTS[V_PACKED_CTA].cap)
@@ -221,8 +233,8 @@ __global__ void __launch_bounds__(256) k_bin_rows(DevCsr A, DevCsr M, const int6
             w = work[r];
             if (mlen == 0 || w == 0) {
                 bin[r] = BIN_SKIP;
-            } else if (pack != PACK_NONE && packed_bin(pack, mlen, alen, w, M.n) != BIN_SKIP) {
-                bin[r] = packed_bin(pack, mlen, alen, w, M.n);
+            } else if (pack != PACK_NONE && packed_bin(pack, mlen, alen, w, maxb[r], M.n) != BIN_SKIP) {
+                bin[r] = packed_bin(pack, mlen, alen, w, maxb[r], M.n);
             } else {
                 const int qm = min(NB_M - 1, ilog2_u64(static_cast<unsigned long long>(mlen)));
                 const int qb = min(NB_B - 1, ilog2_u64(static_cast<unsigned long long>(w / alen)));
@@ -1029,7 +1041,11 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     const bool free_choice = rq.force_variant < 0 && rq.force_accum == GK_ACCUM_AUTO && !rq.bin_variant &&
                              !rq.stats_only && !rq.bin_stats_out;
     const bool operand_mask = M.col == A.col || M.col == B.col;
-    const int pack = !free_choice ? PACK_NONE : (write && !operand_mask ? PACK_CTA : PACK_WARP);
+    const bool flat = static_cast<double>(A.nnz) / A.m * (static_cast<double>(B.nnz) / B.m) >= PACKED_FLAT_MEAN;
+    const int pack = !free_choice                           ? PACK_NONE
+                     : write                                ? (operand_mask ? PACK_WARP : PACK_CTA)
+                     : rq.sched == GK_SCHED_LEARNED         ? (flat ? PACK_FLAT : PACK_NONE)
+                                                            : PACK_WARP;
     k_bin_rows<<<sms * 2, 256, 0, s>>>(A, M, work, maxb, bin, bins, pack, gate);
     GK_CUDA(cudaGetLastError());
     if (rq.bin_variant) {
