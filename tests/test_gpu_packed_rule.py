@@ -51,3 +51,16 @@ def test_written_values_learned(gk, orc, cuda, n):
     M = rows_csr(n, [x for x, _ in lens], 3, values=False)
     got = gk.mxmm_masked(A.to("cuda"), B.to("cuda"), M.to("cuda"), sched="learned").cpu().numpy()
     np.testing.assert_array_equal(got, orc.mxmm(A, B, M))
+
+
+def test_copies_of_an_operand_are_one_mask(gk, orc, cuda):
+    """The mask is recognised as an operand in host arrays, which are staged one by
+    one, and in copies: no CTA kind for triangles."""
+    L = gk.lower_host(gk.gen_rmat(11, 16, seed=3))
+    want = orc.mxmm(L, L, L)
+    D = L.to("cuda")
+    copy = L.to("cuda")
+    for args in ((D, D, D), (D, D, copy), (L, L, L)):
+        got, names = kernels(lambda: gk.mxmm_masked(*args, sched="learned"))
+        np.testing.assert_array_equal(got.cpu().numpy() if hasattr(got, "cpu") else got, want)
+        assert not any("k_packed_cta" in x for x in names)
