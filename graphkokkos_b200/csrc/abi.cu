@@ -84,9 +84,29 @@ struct CopyPipe {
     }
 };
 
-// The engine's product C<L> = L·L over the given order.
-static int tc_engine(const DevCsr &d, int epi, unsigned long long *dev_sums, int sched, cudaStream_t s, Scratch &scr,
-                     int force_variant = -1) {
+// A product of one matrix with itself, under itself, its content check queued in
+// front of it: one synchronisation for the check and the plan.
+int run_spgemm_checked(SpgemmRequest &rq, const char *name, Scratch &scr) {
+    const DevCsr d = rq.A;
+    const cudaStream_t s = rq.stream;
+    if (!csr_check_active(s)) return run_spgemm(rq, scr);
+    if (rq.force_variant < 0 && sched_prepare(rq.sched, rq.force_accum) != GK_OK) {
+        GK_CHECK(check_csr(d, CSR_SORTED, name, s, scr));  // a defect comes before a mode that does not fit
+        return run_spgemm(rq, scr);
+    }
+    CsrCheckOut *chk;
+    GK_CHECK(scr.alloc(&chk, 1));
+    GK_CUDA(cudaMemsetAsync(chk, 0, sizeof(CsrCheckOut), s));
+    GK_CHECK(launch_csr_check(d, CSR_SORTED, chk, s));
+    rq.checks = chk;
+    rq.nchecks = 1;
+    const int status = run_spgemm(rq, scr);
+    if (status == GK_ERR_INVALID_CSR) GK_CHECK(check_csr(d, CSR_SORTED, name, s, scr));  // names the defect
+    return status;
+}
+
+static SpgemmRequest tc_request(const DevCsr &d, int epi, unsigned long long *dev_sums, int sched, cudaStream_t s,
+                                int force_variant = -1) {
     SpgemmRequest rq;
     rq.A = rq.B = rq.M = d;
     rq.epi = epi;
@@ -95,15 +115,21 @@ static int tc_engine(const DevCsr &d, int epi, unsigned long long *dev_sums, int
     rq.sums = dev_sums;
     rq.stream = s;
     rq.force_variant = force_variant;
-    return run_spgemm(rq, scr);
+    return rq;
+}
+
+// The engine's product C<L> = L·L over the given order.
+static int tc_engine(const DevCsr &d, int epi, unsigned long long *dev_sums, int sched, cudaStream_t s, Scratch &scr) {
+    return run_spgemm(tc_request(d, epi, dev_sums, sched, s), scr);
 }
 
 static int tc_common(const gk_csr *L, int epi, unsigned long long *dev_sums, int sched, cudaStream_t s,
                      Scratch &scr, int force_variant = -1) {
     DevCsr d;
-    GK_CHECK(stage_csr(L, &d, scr, s, nullptr, CSR_SORTED, "L"));
+    GK_CHECK(stage_csr(L, &d, scr, s, nullptr, 0, "L"));
     d.val = nullptr;  // plus-pair: an adjacency pattern
-    return tc_engine(d, epi, dev_sums, sched, s, scr, force_variant);
+    SpgemmRequest rq = tc_request(d, epi, dev_sums, sched, s, force_variant);
+    return run_spgemm_checked(rq, "L", scr);
 }
 
 // ---- batched graphs: block-diagonal concatenation -------------------------------
@@ -447,20 +473,15 @@ int gk_tc_vertex(const gk_csr *A, int32_t *counts, int sched, void *stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Scratch scr(s);
     DevCsr d;
-    GK_CHECK(stage_csr(A, &d, scr, s, nullptr, CSR_SORTED, "A"));
+    GK_CHECK(stage_csr(A, &d, scr, s, nullptr, 0, "A"));
     d.val = nullptr;
     unsigned long long *sums;
     int32_t *out;
     GK_CHECK(scr.alloc(&sums, A->m + 1));
     GK_CHECK(scr.alloc(&out, A->m));
     GK_CUDA(cudaMemsetAsync(sums, 0, sizeof(unsigned long long) * (A->m + 1), s));
-    SpgemmRequest rq;
-    rq.A = rq.B = rq.M = d;
-    rq.epi = EPI_KEYED;  // row sums of C<A> = A·A
-    rq.sched = sched;
-    rq.sums = sums;
-    rq.stream = s;
-    GK_CHECK(run_spgemm(rq, scr));
+    SpgemmRequest rq = tc_request(d, EPI_KEYED, sums, sched, s);  // row sums of C<A> = A·A
+    GK_CHECK(run_spgemm_checked(rq, "A", scr));
     k_half_int<<<ceil_div(A->m, 256), 256, 0, s>>>(A->m, sums, out);
     note_launches(1);
     GK_CUDA(cudaGetLastError());

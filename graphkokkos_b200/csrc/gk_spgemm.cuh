@@ -41,6 +41,8 @@ struct SpgemmRequest {
 };
 
 int run_spgemm(const SpgemmRequest &req, Scratch &scr);
+// The same for A = B = M, not yet checked, with its content check (abi.cu).
+int run_spgemm_checked(SpgemmRequest &req, const char *name, Scratch &scr);
 
 // Everything run_spgemm configures on its first use (kernel attributes and
 // grid sizes of every variant for this epilogue, the learned model's upload),

@@ -5,10 +5,11 @@
 // memory (a cudaMalloc from us would fail, or fragment and stall their pool),
 // or a host that forbids its plugins from allocating inside its processing loop
 // because an allocation can synchronise the device.  For them this entry point
-// runs the same masked-SpGEMM triangle count as gk_tc_count, but every scratch
-// buffer (the scheduler's per-row plan, the scan's temporary storage and the
-// count accumulator) is carved from one fixed array in device memory declared
-// below, instead of being allocated per call.
+// gives gk_tc_count's result by the masked-SpGEMM engine over the given order (the
+// degree order's scratch grows with the edges, which a fixed array cannot hold):
+// every scratch buffer (the scheduler's per-row plan, the scan's temporary storage
+// and the count accumulator) is carved from one fixed array in device memory
+// declared below, instead of being allocated per call.
 //
 //  * The array is a file-scope __device__ variable of GK_NOALLOC_BYTES
 //    (36 MiB): every GPU on which this library is loaded holds it until the
@@ -20,8 +21,9 @@
 //    time the entry point is called on a device (with that device current);
 //    that first call should therefore come before any stream capture.
 //  * L goes through the same content check as every entry point (row
-//    pointers, column range, sorted rows), which synchronises the stream once;
-//    GK_CHECK_CSR=0 skips it for trusted input.
+//    pointers, column range, sorted rows), whose result is read together with the
+//    plan's (one synchronisation of the stream); GK_CHECK_CSR=0 skips both for
+//    trusted input.
 //  * All calls share the array and it keeps the last call's contents; what
 //    must start at zero is cleared by each call.  Calls whose work overlaps on
 //    the GPU (other host threads, or other streams without ordering between
@@ -84,14 +86,13 @@ extern "C" int gk_tc_count_noalloc(const gk_csr *L, uint64_t *count, int sched, 
     GK_CHECK(scr.alloc(&d, 1));
     GK_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned long long), s));
     DevCsr dl{L->m, L->n, L->nnz, L->rowptr, L->col, nullptr};
-    GK_CHECK(check_csr(dl, CSR_SORTED, "L", s, scr));
     SpgemmRequest rq;
     rq.A = rq.B = rq.M = dl;
     rq.epi = EPI_SUM;
     rq.sched = sched;
     rq.sums = d;
     rq.stream = s;
-    GK_CHECK(run_spgemm(rq, scr));
+    GK_CHECK(run_spgemm_checked(rq, "L", scr));
     if (is_device_pointer(count)) {
         GK_CUDA(cudaMemcpyAsync(count, d, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
     } else {

@@ -1044,11 +1044,13 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     // (by shape and number of entries: the arrays may be copies, staged ones, too)
     auto like_mask = [&](const DevCsr &x) { return x.m == M.m && x.n == M.n && x.nnz == M.nnz; };
     const bool operand_mask = like_mask(A) || like_mask(B);
+    // (a captured sum launches every kernel anyway: the model's choice alone)
     const bool flat = static_cast<double>(A.nnz) / A.m * (static_cast<double>(B.nnz) / B.m) >= PACKED_FLAT_MEAN;
     const int pack = !free_choice                           ? PACK_NONE
                      : write                                ? (operand_mask ? PACK_WARP : PACK_CTA)
-                     : rq.sched == GK_SCHED_LEARNED         ? (flat ? PACK_FLAT : PACK_NONE)
+                     : rq.sched == GK_SCHED_LEARNED         ? (flat && csr_check_active(s) ? PACK_FLAT : PACK_NONE)
                                                             : PACK_WARP;
+    const bool packed_kinds = pack != PACK_NONE || (rq.sched == GK_SCHED_PLAIN && rq.force_accum == GK_ACCUM_AUTO);
     k_bin_rows<<<sms * 2, 256, 0, s>>>(A, M, work, maxb, bin, bins, pack, gate);
     GK_CUDA(cudaGetLastError());
     if (rq.bin_variant) {
@@ -1083,10 +1085,10 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     // Which variants have rows: read back together with the pending checks, so
     // that only those are launched (an empty persistent grid costs 2 to 10 us,
     // and there are 24).  Inside a capture, or with the checks switched off (the
-    // call is then asynchronous), all of them are.
+    // call is then asynchronous), all of them are; a forced variant needs no look.
     int hoff[NK + 1];
     bool known = false;
-    if (csr_check_active(s)) {
+    if (csr_check_active(s) && (gate.n || rq.force_variant < 0)) {
         GK_CUDA(cudaMemcpyAsync(hoff, voff, sizeof(hoff), cudaMemcpyDeviceToHost, s));
         if (gate.n)
             GK_CUDA(cudaMemcpyAsync(hchk, gate.chk, sizeof(CsrCheckOut) * gate.n, cudaMemcpyDeviceToHost, s));
@@ -1133,7 +1135,8 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
         GK_CUDA(cudaEventRecord(tev[0], s));
     }
     for (int v = 0; v < NK; ++v) {
-        if ((rq.force_variant >= 0 && v != rq.force_variant) || (known && hoff[v] == hoff[v + 1])) {
+        if ((rq.force_variant >= 0 && v != rq.force_variant) || (known && hoff[v] == hoff[v + 1]) ||
+            (v >= NV && !packed_kinds)) {
             if (timed) GK_CUDA(cudaEventRecord(tev[v + 1], s));
             continue;
         }

@@ -28,7 +28,8 @@
  *    gk_bc_batch, whose order does not matter) columns strictly increasing
  *    within each row.  A violation returns GK_ERR_INVALID_CSR naming the
  *    matrix, the defect and the first bad row.  The check reads the result on
- *    the host (one synchronisation of `stream`); it is skipped inside a
+ *    the host (one synchronisation of `stream`, with which the masked products
+ *    also learn which of their kernels have rows); it is skipped inside a
  *    stream capture and when the environment sets GK_CHECK_CSR=0, in which
  *    case the caller guarantees well-formed input.
  *  - Results are bit-exact with the reference on the same inputs: integer
@@ -112,7 +113,8 @@ int gk_mxmm_masked(const gk_csr *A, const gk_csr *B, const gk_csr *M, int32_t *C
  * Small and flat graphs are counted entry by entry, other strict lower
  * triangles in degree order (csrc/tri.cu), without the row-bin scheduler; other
  * square patterns, and calls inside a stream capture, by the engine's product.
- * Outside a capture the call synchronises `stream` once to choose.
+ * Outside a capture the call synchronises `stream` once to choose, and once
+ * more where the engine's product is chosen.
  * *count receives the uint64 total (the reference returns int64). */
 int gk_tc_count(const gk_csr *L, uint64_t *count, int sched, void *stream);
 
