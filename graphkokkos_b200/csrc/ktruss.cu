@@ -193,6 +193,15 @@ __global__ void k_keep_sym(int64_t m, int64_t cap, const int64_t *rp, const int3
     for (int64_t p = nnz + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p <= cap; p += stride) keep[p] = 0;
 }
 
+// keep[p] for every entry off the diagonal.
+__global__ void k_keep_edges(int64_t m, int64_t cap, const int64_t *rp, const int32_t *col, const int32_t *row,
+                             int32_t *keep) {
+    const int64_t nnz = rp[m];
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p <= cap; p += stride)
+        keep[p] = p < nnz && row[p] != col[p];
+}
+
 struct KtBuffers {
     int64_t m, cap;            // rows, nnz of the input (capacity of every edge array)
     int64_t *rp, *nrp;         // current / pruned row pointers
@@ -612,6 +621,7 @@ int ktruss_device(int64_t m, int64_t nnz0, int64_t *rp_a, int32_t *col_a, int k,
     b.k = k;
     b.sched = sched;
     GK_CHECK(scr.alloc(&b.row, nnz0));
+    bool loops = false;  // self-loops of a symmetric pattern
     {
         SymFacts *facts, h{};
         GK_CHECK(scr.alloc(&facts, 1));
@@ -621,8 +631,11 @@ int ktruss_device(int64_t m, int64_t nnz0, int64_t *rp_a, int32_t *col_a, int k,
         note_launches(2);
         GK_CUDA(cudaMemcpyAsync(&h, facts, sizeof(h), cudaMemcpyDeviceToHost, s));
         GK_CUDA(cudaStreamSynchronize(s));
-        b.sym = h.symmetric(nnz0);
-        if (b.sym && h.diagonal == 0) {
+        // the supports on the lower triangle leave self-loops out, which the product
+        // counts (a loop at i supports every edge of i): those take the full mask
+        b.sym = h.symmetric(nnz0) && h.diagonal == 0;
+        loops = h.symmetric(nnz0) && h.diagonal > 0;
+        if (b.sym) {
             bool done = false;
             GK_CHECK(sched_prepare(sched, GK_ACCUM_AUTO));
             GK_CHECK(ktruss_peel(m, nnz0, rp_a, col_a, b.row, k, iters_out, nnz_out, rp_res, col_res, s, scr, &done));
@@ -678,6 +691,20 @@ int ktruss_device(int64_t m, int64_t nnz0, int64_t *rp_a, int32_t *col_a, int k,
     }
     *iters_out = static_cast<int>(h.iters);
     *nnz_out = h.kept;
+    if (!loops) return GK_OK;
+    // the truss of an undirected graph has no loops
+    const int sms = ctx().num_sms;
+    size_t scan_bytes = b.scan_bytes;
+    k_row_of<<<sms * 8, 256, 0, s>>>(m, b.rp, b.row);
+    k_keep_edges<<<sms * 8, 256, 0, s>>>(m, b.cap, b.rp, b.col, b.row, b.keep);
+    GK_CUDA(cub::DeviceScan::ExclusiveSum(b.scan_tmp, scan_bytes, b.keep, b.pos, b.cap + 1, s));
+    k_compact<<<sms * 8, 256, 0, s>>>(m, b.rp, b.col, b.keep, b.pos, b.nrp, b.ncol);
+    note_launches(3);
+    GK_CUDA(cudaGetLastError());
+    GK_CUDA(cudaMemcpyAsync(nnz_out, b.pos + nnz0, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    GK_CUDA(cudaStreamSynchronize(s));
+    *rp_res = b.nrp;
+    *col_res = b.ncol;
     return GK_OK;
 }
 

@@ -196,7 +196,9 @@ int gk_tc_count_batched(const gk_csr *graphs, int ngraphs, uint64_t *counts, int
  * keep the entries with S >= k-2, until nnz stops changing (k_truss,
  * src/main.cpp:94-141, with its View-size defect at :99/:118 not
  * reproduced).  On return inout->rowptr/col/nnz hold the truss and *iters the
- * number of passes (the reference's "Iterations:" line, :138).  k >= 3. */
+ * number of passes (the reference's "Iterations:" line, :138).  k >= 3.
+ * Self-loops of a symmetric matrix count in the supports, as the product counts
+ * them, but are no part of the truss. */
 int gk_ktruss(gk_csr_mut *inout, int k, int *iters, int sched, void *stream);
 
 /* Batched betweenness centrality in FP64 over the given sources:
