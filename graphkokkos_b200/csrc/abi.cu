@@ -718,7 +718,6 @@ int gk_tc_count_batched(const gk_csr *graphs, int ngraphs, uint64_t *counts, int
         in.vbase = v0;
         in.key = key;
         in.gvbase = dvbase;
-        in.key0 = 0;
         in.nkeys = ngraphs;
         for (int g = g0; g < g1; ++g) in.max_m = std::max(in.max_m, slots[g].m);
         bool done = false;

@@ -432,7 +432,7 @@ static int cmask_by_sort(const CmaskArgs &a, cudaStream_t s, Scratch &scr) {
 
 template <bool FILL>
 static int launch_rows(const CmaskArgs &a, cudaStream_t s) {
-    // the longest rows first
+    // the class of the longest rows first
     if (FILL && a.win <= CM_DENSE_WIN) GK_CHECK((launch_map<256, FILL, FILL>(a, s)));
     else if (a.win <= CM_SMALL_WIN) GK_CHECK((launch_map<128, FILL, false>(a, s)));
     else GK_CHECK((launch_map<512, FILL, false>(a, s)));

@@ -51,7 +51,7 @@ struct TriInput {
     int64_t ebase = 0, vbase = 0;
     const int32_t *key = nullptr;    // batch: graph of vertex vbase + r
     const int64_t *gvbase = nullptr; // batch: first vertex of every graph
-    int key0 = 0, nkeys = 1;         // graphs key0 .. key0 + nkeys - 1 occur
+    int nkeys = 1;                   // graphs of the batch
     int64_t max_m = 0;               // vertices of the largest of them
 };
 

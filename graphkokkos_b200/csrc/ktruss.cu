@@ -320,7 +320,6 @@ static int while_graph(cudaStream_t s, int *launches_per_pass, F pass) {
 struct PeelState {
     unsigned int pass, iters, done, fetch;
     unsigned int n[2];           // edges of pass t at [t & 1], of pass t + 1 at the other
-    unsigned long long removed;  // edges over all passes
 };
 
 struct PeelArgs {
@@ -453,7 +452,6 @@ __global__ void k_peel_end(PeelState *st, unsigned int max_iters) {
     if (st->done) return;
     const unsigned int t = st->pass, n = st->n[t & 1];
     st->iters = t;
-    st->removed += n;
     if (n > 0 && t < max_iters) {
         st->n[t & 1] = 0;
         st->fetch = 0;

@@ -207,9 +207,10 @@ __global__ void k_row_stats(DevCsr A, const int32_t *__restrict__ blen, int64_t 
     }
 }
 
-// Bin of every row (a packed kind's where `pack` is set and the row is for it) and the bins' statistics: the rows of a bin among a warp's 32 are
-// summed by shuffles first (rows side by side mostly share a bin; one 64-bit
-// shared-memory atomic per row and value took 30 us for 20,000 rows).
+// Bin of every row (a packed kind's where `pack` is set and the row is for it) and
+// the bins' statistics: the rows of a bin among a warp's 32 are summed by shuffles
+// first (rows side by side mostly share a bin; one 64-bit shared-memory atomic per
+// row and value took 30 us for 20,000 rows).
 __global__ void __launch_bounds__(256) k_bin_rows(DevCsr A, DevCsr M, const int64_t *work, const int32_t *maxb,
                                                   uint16_t *bin, BinStats *bins, int pack, Gate gate) {
     if (!gate.open()) return;

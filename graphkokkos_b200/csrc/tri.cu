@@ -71,13 +71,13 @@ __global__ void __launch_bounds__(256) k_tri_col_counts(DevCsr L, int64_t ebase,
 
 // Sort key of every vertex: its graph, then descending degree.
 template <class KeyT>
-__global__ void __launch_bounds__(256) k_tri_vertex_keys(DevCsr L, int64_t vbase, const int32_t *key, int key0,
-                                                         int dbits, const uint32_t *cnt, KeyT *vkey, uint32_t *iota) {
+__global__ void __launch_bounds__(256) k_tri_vertex_keys(DevCsr L, int64_t vbase, const int32_t *key, int dbits,
+                                                         const uint32_t *cnt, KeyT *vkey, uint32_t *iota) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < L.m; r += stride) {
         const uint32_t d = cnt[r] + static_cast<uint32_t>(L.rp[r + 1] - L.rp[r]);
         KeyT k = (KeyT(1) << dbits) - 1 - d;
-        if (key) k |= static_cast<KeyT>(key[vbase + r] - key0) << dbits;
+        if (key) k |= static_cast<KeyT>(key[vbase + r]) << dbits;
         vkey[r] = k;
         iota[r] = static_cast<uint32_t>(r);
     }
@@ -562,7 +562,7 @@ __device__ __forceinline__ uint32_t warp_incl_sum(uint32_t x, int lane) {
     return x;
 }
 
-// First lane whose inclusive count exceeds u (32 when none does).
+// First lane whose inclusive count exceeds u (31 when none does).
 __device__ __forceinline__ int warp_find(uint32_t incl, uint32_t u) {
     int j = 0;
 #pragma unroll
@@ -748,13 +748,13 @@ struct TriSupArgs {
 // many warps an SM otherwise; the sums in shared memory are 16-bit for the same
 // reason (11 -> 9 KB an item, 3.75 -> 3.3 ms).
 constexpr int TRI_SUP_ACC = 1024;  // places kept in shared memory; the others take an atomic per hit
-template <int LB>
+constexpr int TRI_SUP_LB = 15;     // log2 bits of the bitmap
 __global__ void __launch_bounds__(64) k_tri_support(TriSupArgs sa) {
     const TriArgs &p = sa.t;
     int32_t *sup = sa.sup;
     constexpr unsigned FULL = 0xFFFFFFFFu;
-    constexpr int NT = 64, BW = 1 << (LB - 5), FW = 1 << (TRI_FB - 5), PER = BW / NT;
-    constexpr uint32_t PAD = (1u << LB) - 1;
+    constexpr int NT = 64, BW = 1 << (TRI_SUP_LB - 5), FW = 1 << (TRI_FB - 5), PER = BW / NT;
+    constexpr uint32_t PAD = (1u << TRI_SUP_LB) - 1;
     __shared__ __align__(16) uint32_t bm[BW];
     __shared__ __align__(16) uint16_t pre[BW];  // columns of row k in the words before
     // acc: two 16-bit sums a word (an item's entries, at most `chunk` = 2,048, hit a place once each)
@@ -1364,7 +1364,7 @@ static int vertex_order(const TriInput &in, int dbits, int gbits, const uint32_t
     KeyT *vkey, *vkey2;
     GK_CHECK(scr.alloc(&vkey, m));
     GK_CHECK(scr.alloc(&vkey2, m));
-    k_tri_vertex_keys<KeyT><<<ctx().num_sms * 8, 256, 0, s>>>(in.L, in.vbase, in.key, in.key0, dbits, cnt, vkey, iota);
+    k_tri_vertex_keys<KeyT><<<ctx().num_sms * 8, 256, 0, s>>>(in.L, in.vbase, in.key, dbits, cnt, vkey, iota);
     note_launches(2);
     GK_CUDA(cudaGetLastError());
     size_t vb = 0;
@@ -1468,7 +1468,7 @@ static int order_vertices(const TriInput &in, uint32_t **deg, uint32_t **rank, c
     GK_CHECK(scr.alloc(rank, m));
     GK_CHECK(scr.alloc(deg, m));
     GK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * m, s));
-    const int cc = static_cast<int>(std::max<int64_t>(sms * 8, in.L.nnz >> 15));
+    const int cc = static_cast<int>(std::max<int64_t>(sms * 8, (in.L.nnz + (1 << 15) - 1) >> 15));
     k_tri_col_counts<<<cc, 256, 0, s>>>(in.L, in.ebase, in.vbase, cnt);
     const int dbits = bits_for(in.key ? in.max_m : m), gbits = in.key ? bits_for(in.nkeys) : 0;
     if (dbits + gbits <= 32) GK_CHECK(vertex_order<uint32_t>(in, dbits, gbits, cnt, iota, perm, s, scr));
@@ -1526,11 +1526,11 @@ int tri_support(const DevCsr &L, TriSupport *out, cudaStream_t s, Scratch &scr, 
     GK_CHECK(scr.alloc(&out->sup, out->numbers));
     GK_CUDA(cudaMemsetAsync(out->sup, 0, sizeof(int32_t) * out->numbers, s));
     TriSupArgs a;
-    GK_CHECK(orient(in, deg, rank, 15, true, &a.t, s, scr));
+    GK_CHECK(orient(in, deg, rank, TRI_SUP_LB, true, &a.t, s, scr));
     a.sup = out->sup;
     int per_sm = 0;
-    GK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tri_support<15>, 64, 0));
-    k_tri_support<15><<<ctx().num_sms * std::max(per_sm, 1), 64, 0, s>>>(a);
+    GK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tri_support, 64, 0));
+    k_tri_support<<<ctx().num_sms * std::max(per_sm, 1), 64, 0, s>>>(a);
     note_launches(1);
     GK_CUDA(cudaGetLastError());
     out->g = a.t.g;

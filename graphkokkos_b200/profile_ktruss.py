@@ -4,10 +4,11 @@
 
 Builds the seeded RMAT graph on the device and calls gk_ktruss --reps times
 after --warmup calls, printing one JSON line with the per-call CUDA-event time
-and the per-variant profile (gk_prof_*) of one extra call.  With
---host-passes the pass loop is driven from the host (library profiling mode
-2), so that every kernel of every pass is a separate launch an ncu capture can
-select; without it the passes run as one CUDA graph.
+and the per-variant profile (gk_prof_*) of one extra call.  The
+graph is undirected and takes the peeling passes, whose kernels are separate
+launches in any case; --host-passes (library profiling mode 2) brackets the product
+loop's launches with events where that loop runs (patterns that are not symmetric,
+or no memory for the peeling), and drives its passes from the host.
 """
 import argparse
 import ctypes
