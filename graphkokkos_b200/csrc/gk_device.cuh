@@ -155,28 +155,34 @@ __device__ __forceinline__ int64_t group_lower_bound(const int32_t *__restrict__
     return lo + __popc(bal);
 }
 
+// The row of entry p among the rows [lo, hi] (the first whose end lies beyond it,
+// which exists), by one warp.
+template <class RpT>
+__device__ __forceinline__ int64_t warp_row_of(const RpT *__restrict__ rp, int64_t lo, int64_t hi, int64_t p, int lane) {
+    while (lo < hi) {
+        const int64_t len = hi - lo;
+        const int64_t piv = lo + len * lane / 32;
+        // pivots ending at or before p
+        const int c = __popc(__ballot_sync(0xFFFFFFFFu, static_cast<int64_t>(__ldg(rp + piv + 1)) <= p));
+        const int64_t nlo = c == 0 ? lo : lo + len * (c - 1) / 32 + 1;
+        hi = c == 32 ? hi : lo + len * c / 32;
+        lo = nlo;
+    }
+    return lo;
+}
+
 // Walks the entries [p0, p1) of a CSR with one warp, 32 at a time whatever the
 // lengths of the rows: f(p, row, leader, peers, on) with the lanes' consecutive
 // entries p, their rows, the first lane and the lanes of the same row among
 // those the call covers (on).  The ends of 32 consecutive rows are held one
 // per lane and searched by shuffles, so a hub row is as many steps as its
-// entries need and runs of empty rows cost one window each.
+// entries need; a run of more than 32 empty rows is passed by a search (few edges
+// on many vertices: 3,000 entries in 460,000 rows, a count 388 -> 103 us).
 template <class RpT, class F>
 __device__ __forceinline__ void walk_entries(const RpT *__restrict__ rp, int64_t m, int64_t p0, int64_t p1,
                                              int lane, F f) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
-    // first row whose end lies beyond p0
-    int64_t lo = 0, hi = m - 1;
-    while (hi - lo > 0) {
-        const int64_t len = hi - lo;
-        const int64_t piv = lo + len * lane / 32;
-        const unsigned c = __popc(__ballot_sync(FULL, static_cast<int64_t>(__ldg(rp + piv + 1)) <= p0));  // pivots ending at or before p0
-        const int64_t nlo = c == 0 ? lo : lo + len * (c - 1) / 32 + 1;
-        const int64_t nhi = c == 32 ? hi : lo + len * c / 32;
-        lo = nlo;
-        hi = nhi;
-    }
-    int64_t r = lo;
+    int64_t r = warp_row_of(rp, 0, m - 1, p0, lane);
     int64_t end = r + lane < m ? static_cast<int64_t>(__ldg(rp + r + lane + 1)) : p1;
     for (int64_t base = p0; base < p1; base += 32) {
         const int64_t p = base + lane;
@@ -196,7 +202,7 @@ __device__ __forceinline__ void walk_entries(const RpT *__restrict__ rp, int64_t
                 todo &= ~onm;
             }
             if (todo) {
-                r += 32;
+                r = onm ? r + 32 : warp_row_of(rp, r + 32, m - 1, base + __ffs(todo) - 1, lane);
                 end = r + lane < m ? static_cast<int64_t>(__ldg(rp + r + lane + 1)) : p1;
             }
         }

@@ -995,17 +995,8 @@ __global__ void __launch_bounds__(32 * TRI_SMALL_WARPS) k_tri_small(DevCsr L, in
     const int64_t step = (int64_t)gridDim.x * TRI_SMALL_WARPS * 32;
     for (int64_t p0 = ((int64_t)blockIdx.x * TRI_SMALL_WARPS + warp) * 32; p0 < L.nnz; p0 += step) {
         const int64_t p1 = min(p0 + 32, L.nnz);
-        // the row of entry p0: the first whose end lies beyond it
-        int64_t lo = 0, hi = L.m - 1;
-        while (lo < hi) {
-            const int64_t len = hi - lo, piv = lo + len * lane / 32;
-            const int c = __popc(__ballot_sync(FULL, __ldg(L.rp + piv + 1) <= p0));
-            const int64_t nlo = c == 0 ? lo : lo + len * (c - 1) / 32 + 1;
-            hi = c == 32 ? hi : lo + len * c / 32;
-            lo = nlo;
-        }
         uint32_t cnt = 0;
-        int64_t r = lo, r0 = __ldg(L.rp + r);
+        int64_t r = warp_row_of(L.rp, 0, L.m - 1, p0, lane), r0 = __ldg(L.rp + r);
         for (int64_t p = p0; p < p1; ++r) {
             const int64_t r1 = __ldg(L.rp + r + 1), e = min(r1, p1);
             if (e > p) {
@@ -1055,6 +1046,15 @@ __global__ void __launch_bounds__(32 * TRI_SMALL_WARPS) k_tri_small(DevCsr L, in
                 __syncwarp();
                 for (int64_t q = r0 + lane; q < r1; q += 32) bm[__ldg(L.col + q) >> 5] = 0;
                 __syncwarp();
+            } else {
+                // an empty row: the next 32 rows at once, behind more of them a search
+                // (63 edges on 10,856 vertices, row by row 661 us, so 62)
+                const int64_t q = r + 1 + lane;
+                const int c = __popc(__ballot_sync(FULL, q < L.m && __ldg(L.rp + q + 1) <= p));
+                if (c < 32) r += c;
+                else r = warp_row_of(L.rp, r + 33, L.m - 1, p, lane) - 1;
+                r0 = p;
+                continue;
             }
             r0 = r1;
         }
