@@ -47,16 +47,21 @@ __global__ void __launch_bounds__(NT, block_min_ctas(NT, KIND, CAP, FLOG, LOWB, 
     if (begin == end) return;
     const int nsimple = p.vsimple[p.v];
     const int64_t ibeg = p.item_ex[begin], iend = p.item_ex[end];
+    // NB items a fetch; with few of them one, since they are then the rows that no
+    // smaller kind took, and a CTA would hold several long ones back (412 x 4,459 x 51
+    // with one row of 40,000 products, plain: 1.64 -> 1.07 ms)
+    const int64_t each = (iend - ibeg) / (4 * static_cast<int64_t>(gridDim.x));
+    const int nb = each < 1 ? 1 : (each < NB ? static_cast<int>(each) : NB);
     if (threadIdx.x == 0) s_left = 0;
     unsigned long long local = 0;
 
     while (true) {
         if (threadIdx.x == 0) {
             if (s_left == 0) {
-                s_base = static_cast<int64_t>(atomicAdd(p.fetch + p.v, static_cast<unsigned>(NB)));
-                s_left = NB;
+                s_base = static_cast<int64_t>(atomicAdd(p.fetch + p.v, static_cast<unsigned>(nb)));
+                s_left = nb;
             }
-            const int64_t rel = s_base + (NB - s_left);
+            const int64_t rel = s_base + (nb - s_left);
             --s_left;
             const int64_t I = ibeg + rel;
             s_item = I;
