@@ -1427,16 +1427,15 @@ static int bc_device(BcBuffers &g, const BcFacts &f, const int32_t *src, int nsr
         GK_CHECK(heavy_finish(g.AT, &g.hAT, h, s, scr));
     }
     GK_CUDA(cudaMemsetAsync(bc, 0, sizeof(double) * A.m, s));
-    // the device's free memory is asked for only where the widest chunk is large
-    size_t free_b = ~size_t(0) / 4, total_b = 0;
-    if ((double)A.m * 32 * GK_BC_TMAX * 16 > double(1 << 28)) cudaMemGetInfo(&free_b, &total_b);
     int widest = GK_BC_TMAX;
     for (int done = 0; done < nsrc;) {
         const int left = nsrc - done;
         int T = widest;
         while (T > 1 && 32 * (T / 2) >= left) T /= 2;
-        // two FP64 m x W arrays must fit comfortably
-        while (T > 1 && (double)A.m * 32 * T * 16 > 0.6 * (double)free_b) T /= 2;
+        // two FP64 m x W arrays must fit the device comfortably; whether they fit what
+        // is free shows when they are allocated (asking, cudaMemGetInfo, now and then
+        // took tens of milliseconds)
+        while (T > 1 && (double)A.m * 32 * T * 16 > 0.6 * (double)ctx().total_mem) T /= 2;
         const int n = left < 32 * T ? left : 32 * T;
         int st;
         switch (T) {
@@ -1447,8 +1446,8 @@ static int bc_device(BcBuffers &g, const BcFacts &f, const int32_t *src, int nsr
             default: st = bc_chunk<1>(g, src + done, n, bc, opt, s); break;
         }
         if (st == GK_ERR_OOM && T > 1) {
-            // no room after all: a chunk allocates before its backward sweep, the
-            // only one to add to the scores, so a narrower one can start over
+            // a chunk allocates before its backward sweep, the only one to add to the
+            // scores, so a narrower one can start over
             scratch_reclaim(s);
             widest = T / 2;
             continue;

@@ -45,6 +45,8 @@ Context &ctx() {
         if (c.device != dev) {
             cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, dev);
             cudaDeviceGetAttribute(&c.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            size_t free_b = 0;
+            cudaMemGetInfo(&free_b, &c.total_mem);  // once per device
             // keep freed stream-ordered scratch cached in the device's default
             // pool instead of returning it to the driver at every sync
             cudaMemPool_t pool;

@@ -42,6 +42,7 @@ struct Context {
     int device = -1;
     int num_sms = 0;
     int max_smem_optin = 0;
+    size_t total_mem = 0;
     bool pool_ready = false;
 };
 // Returns the context of the current device (created on first use).
