@@ -106,11 +106,20 @@ constexpr int64_t PACKED_SHARE = 20;
 // none: 8959 / 8826 / 8824.
 constexpr double PACKED_FLAT_MEAN = 64.0;
 constexpr int64_t PACKED_FLAT_B = 64;
+// Below PACKED_FEW_MEAN products a row on average the plain schedule leaves rows of
+// fewer than PACKED_FEW to the 4-thread groups: a warp is too much for them (us, row
+// sums / L·U count, every row by the rule / so: Erdos-Renyi 1,000,000 (4) 631, 1209 /
+// 418, 970; (8) 769, 1413 / 591, 1374; 300,000 (12), 36 products a row, would lose:
+// 347, 644 / 364, 789).  Under the learned schedule written values keep it (the model
+// has no good variant for them: 634 / 1684 us for L·L under L of the first).
+constexpr double PACKED_FEW_MEAN = 32.0;
+constexpr int64_t PACKED_FEW = 32;
 
 enum : int { PACK_NONE = 0, PACK_FLAT = 1, PACK_WARP = 2, PACK_CTA = 3 };
-__device__ __forceinline__ uint16_t packed_bin(int pack, int64_t mlen, int64_t alen, int64_t work, int64_t maxb,
-                                               int64_t n) {
+__device__ __forceinline__ uint16_t packed_bin(int pack, int64_t least, int64_t mlen, int64_t alen, int64_t work,
+                                               int64_t maxb, int64_t n) {
     const bool sparse = mlen * PACKED_SHARE <= n;
+    if (work < least) return BIN_SKIP;
     if (pack == PACK_FLAT && maxb > PACKED_FLAT_B) return BIN_SKIP;
     if (work <= (sparse ? PACKED_WORK : PACKED_DENSE_WORK) && mlen <= VARIANTS[V_PACKED].cap) return BIN_PACKED;
     if (pack == PACK_CTA && sparse && work <= PACKED_CTA_WORK && work <= PACKED_CTA_MEAN * alen &&
@@ -212,7 +221,8 @@ __global__ void k_row_stats(DevCsr A, const int32_t *__restrict__ blen, int64_t 
 // first (rows side by side mostly share a bin; one 64-bit shared-memory atomic per
 // row and value took 30 us for 20,000 rows).
 __global__ void __launch_bounds__(256) k_bin_rows(DevCsr A, DevCsr M, const int64_t *work, const int32_t *maxb,
-                                                  uint16_t *bin, BinStats *bins, int pack, Gate gate) {
+                                                  uint16_t *bin, BinStats *bins, int pack, int64_t least,
+                                                  Gate gate) {
     if (!gate.open()) return;
     constexpr unsigned FULL = 0xFFFFFFFFu;
     __shared__ unsigned long long s_rows[NBINS], s_m[NBINS], s_a[NBINS], s_w[NBINS];
@@ -235,8 +245,8 @@ __global__ void __launch_bounds__(256) k_bin_rows(DevCsr A, DevCsr M, const int6
             w = work[r];
             if (mlen == 0 || w == 0) {
                 bin[r] = BIN_SKIP;
-            } else if (pack != PACK_NONE && packed_bin(pack, mlen, alen, w, maxb[r], M.n) != BIN_SKIP) {
-                bin[r] = packed_bin(pack, mlen, alen, w, maxb[r], M.n);
+            } else if (pack != PACK_NONE && packed_bin(pack, least, mlen, alen, w, maxb[r], M.n) != BIN_SKIP) {
+                bin[r] = packed_bin(pack, least, mlen, alen, w, maxb[r], M.n);
             } else {
                 const int qm = min(NB_M - 1, ilog2_u64(static_cast<unsigned long long>(mlen)));
                 const int qb = min(NB_B - 1, ilog2_u64(static_cast<unsigned long long>(w / alen)));
@@ -1046,13 +1056,15 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     auto like_mask = [&](const DevCsr &x) { return x.m == M.m && x.n == M.n && x.nnz == M.nnz; };
     const bool operand_mask = like_mask(A) || like_mask(B);
     // (a captured sum launches every kernel anyway: the model's choice alone)
-    const bool flat = static_cast<double>(A.nnz) / A.m * (static_cast<double>(B.nnz) / B.m) >= PACKED_FLAT_MEAN;
+    const double mean = static_cast<double>(A.nnz) / A.m * (static_cast<double>(B.nnz) / B.m);
+    const bool flat = mean >= PACKED_FLAT_MEAN;
+    const int64_t least = rq.sched == GK_SCHED_PLAIN && mean < PACKED_FEW_MEAN ? PACKED_FEW : 0;
     const int pack = !free_choice                           ? PACK_NONE
                      : write                                ? (operand_mask ? PACK_WARP : PACK_CTA)
                      : rq.sched == GK_SCHED_LEARNED         ? (flat && csr_check_active(s) ? PACK_FLAT : PACK_NONE)
                                                             : PACK_WARP;
     const bool packed_kinds = pack != PACK_NONE || (rq.sched == GK_SCHED_PLAIN && rq.force_accum == GK_ACCUM_AUTO);
-    k_bin_rows<<<sms * 2, 256, 0, s>>>(A, M, work, maxb, bin, bins, pack, gate);
+    k_bin_rows<<<sms * 2, 256, 0, s>>>(A, M, work, maxb, bin, bins, pack, least, gate);
     GK_CUDA(cudaGetLastError());
     if (rq.bin_variant) {
         GK_CUDA(cudaMemcpyAsync(var_of_bin, rq.bin_variant, sizeof(int) * NBINS, cudaMemcpyHostToDevice, s));

@@ -64,3 +64,16 @@ def test_copies_of_an_operand_are_one_mask(gk, orc, cuda):
         got, names = kernels(lambda: gk.mxmm_masked(*args, sched="learned"))
         np.testing.assert_array_equal(got.cpu().numpy() if hasattr(got, "cpu") else got, want)
         assert not any("k_packed_cta" in x for x in names)
+
+
+def test_plain_rows_of_a_few_products(gk, orc, cuda):
+    """A product of a few products a row leaves most of them to the groups of four threads
+    (not the rows of 32 products and more)."""
+    L = gk.lower_host(gk.gen_er(50000, 100000, seed=4))
+    D = L.to("cuda")
+    got, names = kernels(lambda: gk.tc_row_sums(D))
+    np.testing.assert_array_equal(got.cpu().numpy().astype(np.uint64), orc.tc_row_sums(L))
+    assert any("k_group" in x for x in names)
+    got, names = kernels(lambda: gk.mxmm_masked(D, D, D))
+    np.testing.assert_array_equal(got.cpu().numpy(), orc.mxmm(L, L, L))
+    assert any("k_group" in x for x in names)
