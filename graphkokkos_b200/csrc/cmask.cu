@@ -401,9 +401,9 @@ static int launch_classes(const CmaskArgs &a, cudaStream_t s) {
 }
 
 // Whether the sort is the better path for these rows: the estimates of both calls'
-// times in us, fitted to the figures below (2^18 columns or fewer: never).  A row in
-// windows costs 0.72 us a window spread over the SMs (clearing, counting and writing
-// 2^14 words) and at least one SM's share of that, 9 us per million products a
+// times in us, fitted to the figures below (2^18 columns or fewer: never).  Windows
+// cost 0.4 ms, a row 0.72 us a window spread over the SMs (clearing, counting and
+// writing 2^14 words) and at least one SM's share of that, 9 us per million products a
 // window, hashed rows 120; the sort 0.8 ms and 260 us per million products, and in
 // every batch of 2^26 products the warp of the longest row is waited for (20 ms per
 // million of its products).  ms, windows / sort, rows x products at columns:
@@ -416,7 +416,7 @@ static bool cm_sorts(const CmaskState &st, int64_t n, int win, int sms) {
     if (st.n[2] == 0) return false;
     const double windows = static_cast<double>((n + (int64_t(1) << win) - 1) >> win);
     const double rows = std::max<double>(st.n[2], sms), work = static_cast<double>(st.work);
-    const double by_windows = windows * (0.72 * rows + 9e-6 * st.long_work) + 1.2e-4 * (work - st.long_work);
+    const double by_windows = 400.0 + windows * (0.72 * rows + 9e-6 * st.long_work) + 1.2e-4 * (work - st.long_work);
     const double batches = std::max(1.0, work / double(1 << 26));
     const double by_sort = 800.0 + 2.6e-4 * work + 2.0 * batches * 0.02 * st.max_work;
     return by_sort < by_windows;
