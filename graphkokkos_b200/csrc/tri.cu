@@ -20,9 +20,9 @@
 // Flat graphs (little work per entry) and small ones keep the given order, in
 // kernels without a plan: k_tri_walk and k_tri_small.
 //
-// RMAT-24 (260 M edges): 274 ms with the engine's product (spgemm.cu), 43 ms
-// here: 23 ms count, 19 ms orientation; RMAT-20: 8.8 -> 1.95 ms; a batch of 409
-// uneven graphs: 37 -> 13 ms.
+// RMAT-24 (260 M edges): 274 ms with the engine's product (spgemm.cu), 42 ms
+// here: 23 ms count, 19 ms orientation; RMAT-20: 8.8 -> 1.9 ms; batches of 409
+// uneven graphs: 34 to 45 -> 12 to 15 ms.
 #include <cub/cub.cuh>
 
 #include <algorithm>
