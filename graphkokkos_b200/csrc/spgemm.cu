@@ -107,13 +107,15 @@ constexpr int64_t PACKED_SHARE = 20;
 constexpr double PACKED_FLAT_MEAN = 64.0;
 constexpr int64_t PACKED_FLAT_B = 64;
 // Below PACKED_FEW_MEAN products a row on average the plain schedule leaves rows of
-// fewer than PACKED_FEW to the 4-thread groups: a warp is too much for them (us, row
+// fewer than PACKED_FEW to the 4-thread groups, where there are enough rows to fill the
+// GPU with warps twenty times over: a warp is too much for them (us, row
 // sums / L·U count, every row by the rule / so: Erdos-Renyi 1,000,000 (4) 631, 1209 /
 // 418, 970; (8) 769, 1413 / 591, 1374; 300,000 (12), 36 products a row, would lose:
 // 347, 644 / 364, 789).  Under the learned schedule written values keep it (the model
-// has no good variant for them: 634 / 1684 us for L·L under L of the first).
+// has no good variant for them: 634 / 1684 us for L·L under L of the first), and few
+// rows are waited for by the row (227 x 1,306 x 8,193 (25, 1, 3), plain: 102 / 350 us).
 constexpr double PACKED_FEW_MEAN = 32.0;
-constexpr int64_t PACKED_FEW = 32;
+constexpr int64_t PACKED_FEW = 32, PACKED_FEW_ROWS = 1 << 17;
 
 enum : int { PACK_NONE = 0, PACK_FLAT = 1, PACK_WARP = 2, PACK_CTA = 3 };
 __device__ __forceinline__ uint16_t packed_bin(int pack, int64_t least, int64_t mlen, int64_t alen, int64_t work,
@@ -1058,7 +1060,8 @@ int run_spgemm(const SpgemmRequest &rq, Scratch &scr) {
     // (a captured sum launches every kernel anyway: the model's choice alone)
     const double mean = static_cast<double>(A.nnz) / A.m * (static_cast<double>(B.nnz) / B.m);
     const bool flat = mean >= PACKED_FLAT_MEAN;
-    const int64_t least = rq.sched == GK_SCHED_PLAIN && mean < PACKED_FEW_MEAN ? PACKED_FEW : 0;
+    const int64_t least =
+        rq.sched == GK_SCHED_PLAIN && mean < PACKED_FEW_MEAN && A.m >= PACKED_FEW_ROWS ? PACKED_FEW : 0;
     const int pack = !free_choice                           ? PACK_NONE
                      : write                                ? (operand_mask ? PACK_WARP : PACK_CTA)
                      : rq.sched == GK_SCHED_LEARNED         ? (flat && csr_check_active(s) ? PACK_FLAT : PACK_NONE)

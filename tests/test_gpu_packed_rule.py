@@ -66,14 +66,15 @@ def test_copies_of_an_operand_are_one_mask(gk, orc, cuda):
         assert not any("k_packed_cta" in x for x in names)
 
 
-def test_plain_rows_of_a_few_products(gk, orc, cuda):
-    """A product of a few products a row leaves most of them to the groups of four threads
-    (not the rows of 32 products and more)."""
-    L = gk.lower_host(gk.gen_er(50000, 100000, seed=4))
+@pytest.mark.parametrize("m,groups", [(131071, False), (131072, True)])
+def test_plain_rows_of_a_few_products(gk, orc, cuda, m, groups):
+    """Of very many rows of a few products each, most are left to the groups of four
+    threads (not the rows of 32 products and more); of fewer, none."""
+    L = gk.lower_host(gk.gen_er(m, 2 * m, seed=4))
     D = L.to("cuda")
     got, names = kernels(lambda: gk.tc_row_sums(D))
     np.testing.assert_array_equal(got.cpu().numpy().astype(np.uint64), orc.tc_row_sums(L))
-    assert any("k_group" in x for x in names)
+    assert any("k_group" in x for x in names) == groups
     got, names = kernels(lambda: gk.mxmm_masked(D, D, D))
     np.testing.assert_array_equal(got.cpu().numpy(), orc.mxmm(L, L, L))
-    assert any("k_group" in x for x in names)
+    assert any("k_group" in x for x in names) == groups
