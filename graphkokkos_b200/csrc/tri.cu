@@ -996,67 +996,71 @@ __global__ void __launch_bounds__(32 * TRI_SMALL_WARPS) k_tri_small(DevCsr L, in
     for (int64_t p0 = ((int64_t)blockIdx.x * TRI_SMALL_WARPS + warp) * 32; p0 < L.nnz; p0 += step) {
         const int64_t p1 = min(p0 + 32, L.nnz);
         uint32_t cnt = 0;
-        int64_t r = warp_row_of(L.rp, 0, L.m - 1, p0, lane), r0 = __ldg(L.rp + r);
-        for (int64_t p = p0; p < p1; ++r) {
-            const int64_t r1 = __ldg(L.rp + r + 1), e = min(r1, p1);
-            if (e > p) {
-                // the rows of the entries p .. e - 1, one per lane
-                const int64_t t = p + lane;
-                int64_t b0 = 0;
-                uint32_t n = 0;
-                if (t < e) {
-                    const int k = __ldg(L.col + t);
-                    b0 = __ldg(L.rp + k);
-                    n = static_cast<uint32_t>(__ldg(L.rp + k + 1) - b0);
+        // the ends of 32 rows, one per lane, and where the first of them starts
+        int64_t r = warp_row_of(L.rp, 0, L.m - 1, p0, lane), first = __ldg(L.rp + r);
+        int64_t end = r + lane < L.m ? __ldg(L.rp + r + lane + 1) : L.nnz;
+        for (int64_t p = p0; p < p1;) {
+            const int past = __popc(__ballot_sync(FULL, end <= p));  // rows that p has passed
+            if (past == 32) {
+                // on to the row of p; behind more than 32 empty rows by a search (63
+                // edges on 10,856 vertices, row by row 661 us, so 62)
+                first = __shfl_sync(FULL, end, 31);
+                r += 32;
+                end = r + lane < L.m ? __ldg(L.rp + r + lane + 1) : L.nnz;
+                if (__shfl_sync(FULL, end, 31) <= p) {
+                    r = warp_row_of(L.rp, r + 32, L.m - 1, p, lane);
+                    first = __ldg(L.rp + r);
+                    end = r + lane < L.m ? __ldg(L.rp + r + lane + 1) : L.nnz;
                 }
-                const uint32_t len = static_cast<uint32_t>(r1 - r0);
-                p = e;
-                if (len > TRI_SMALL_MAP && 8 * __reduce_add_sync(FULL, min(n, 1u << 16)) < len) {
-                    cnt += tri_small_search(L.col, L.col + r0, len, b0, n);
-                    r0 = r1;
-                    continue;
-                }
-                for (int64_t q = r0 + lane; q < r1; q += 32) {
-                    const int x = __ldg(L.col + q);
-                    atomicOr(bm + (x >> 5), 1u << (x & 31));
-                }
-                __syncwarp();
-                const bool longer = tri_small_longer(n, len);
-                if (__any_sync(FULL, longer)) {
-                    cnt += tri_small_search(L.col, L.col + r0, len, b0, longer ? n : 0);
-                    if (longer) n = 0;
-                }
-                const uint32_t u = (n + 3) / 4, incl = warp_incl_sum(u, lane);
-                const uint32_t total = __shfl_sync(FULL, incl, 31);
-                for (uint32_t b = 0; b < total; b += 32) {
-                    const uint32_t at = b + lane;
-                    const int j = warp_find(incl, at) & 31;
-                    const uint32_t z = 4 * (at - __shfl_sync(FULL, incl - u, j));
-                    const uint32_t nj = __shfl_sync(FULL, n, j);
-                    const int64_t bj = __shfl_sync(FULL, b0, j);
-                    if (at < total) {
-#pragma unroll
-                        for (uint32_t c = 0; c < 4; ++c)
-                            if (z + c < nj) {
-                                const uint32_t x = static_cast<uint32_t>(__ldg(L.col + bj + z + c));
-                                cnt += (bm[x >> 5] >> (x & 31)) & 1u;
-                            }
-                    }
-                }
-                __syncwarp();
-                for (int64_t q = r0 + lane; q < r1; q += 32) bm[__ldg(L.col + q) >> 5] = 0;
-                __syncwarp();
-            } else {
-                // an empty row: the next 32 rows at once, behind more of them a search
-                // (63 edges on 10,856 vertices, row by row 661 us, so 62)
-                const int64_t q = r + 1 + lane;
-                const int c = __popc(__ballot_sync(FULL, q < L.m && __ldg(L.rp + q + 1) <= p));
-                if (c < 32) r += c;
-                else r = warp_row_of(L.rp, r + 33, L.m - 1, p, lane) - 1;
-                r0 = p;
                 continue;
             }
-            r0 = r1;
+            const int64_t r1 = __shfl_sync(FULL, end, past), before = __shfl_sync(FULL, end, (past - 1) & 31);
+            const int64_t r0 = past ? before : first, e = min(r1, p1);
+            // the rows of the entries p .. e - 1, one per lane
+            const int64_t t = p + lane;
+            int64_t b0 = 0;
+            uint32_t n = 0;
+            if (t < e) {
+                const int k = __ldg(L.col + t);
+                b0 = __ldg(L.rp + k);
+                n = static_cast<uint32_t>(__ldg(L.rp + k + 1) - b0);
+            }
+            const uint32_t len = static_cast<uint32_t>(r1 - r0);
+            p = e;
+            if (len > TRI_SMALL_MAP && 8 * __reduce_add_sync(FULL, min(n, 1u << 16)) < len) {
+                cnt += tri_small_search(L.col, L.col + r0, len, b0, n);
+                continue;
+            }
+            for (int64_t q = r0 + lane; q < r1; q += 32) {
+                const int x = __ldg(L.col + q);
+                atomicOr(bm + (x >> 5), 1u << (x & 31));
+            }
+            __syncwarp();
+            const bool longer = tri_small_longer(n, len);
+            if (__any_sync(FULL, longer)) {
+                cnt += tri_small_search(L.col, L.col + r0, len, b0, longer ? n : 0);
+                if (longer) n = 0;
+            }
+            const uint32_t u = (n + 3) / 4, incl = warp_incl_sum(u, lane);
+            const uint32_t total = __shfl_sync(FULL, incl, 31);
+            for (uint32_t b = 0; b < total; b += 32) {
+                const uint32_t at = b + lane;
+                const int j = warp_find(incl, at) & 31;
+                const uint32_t z = 4 * (at - __shfl_sync(FULL, incl - u, j));
+                const uint32_t nj = __shfl_sync(FULL, n, j);
+                const int64_t bj = __shfl_sync(FULL, b0, j);
+                if (at < total) {
+#pragma unroll
+                    for (uint32_t c = 0; c < 4; ++c)
+                        if (z + c < nj) {
+                            const uint32_t x = static_cast<uint32_t>(__ldg(L.col + bj + z + c));
+                            cnt += (bm[x >> 5] >> (x & 31)) & 1u;
+                        }
+                }
+            }
+            __syncwarp();
+            for (int64_t q = r0 + lane; q < r1; q += 32) bm[__ldg(L.col + q) >> 5] = 0;
+            __syncwarp();
         }
         local += cnt;
     }
